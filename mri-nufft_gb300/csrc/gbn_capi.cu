@@ -172,13 +172,18 @@ struct gbn_plan_s {
   int nbins = 0;           // bins of the sort
   int64_t bin_bytes = 0;   // device bytes of the per-bin arrays
 
-  // 3D column streaming: the sort is keyed on (x bin, y bin, z cell); the
-  // interp / grad table groups bs2 consecutive z cells (the bins of g), the
-  // spread table cuts each column into chunks of <= kStreamChunk samples
+  // Column streaming: the sort is keyed on the bins of the leading axes and
+  // the first footprint cell of the last one; the interp / grad table groups
+  // bs consecutive keys of the last axis (the bins of g), the spread table
+  // cuts each column into chunks of samples.  With `tc` the spreader is the
+  // tensor-core one, whose 2D table cuts the tiles of bs[0] keys along y.
   int stream_spread = 0;
+  bool tc = false;
   int ngrp = 0;            // interp groups (bins of g)
   int ncol = 0;            // columns
-  int* grp = nullptr;      // group-table scratch, 4 x (ngrp + ncol)
+  int sgrp_k = 0;          // keys of the last axis in a group of the spread table
+  int sgrp_n = 0;          // groups of the spread table
+  int* grp = nullptr;      // group-table scratch, 4 x (ngrp + sgrp_n)
   int* ssub = nullptr;     // spread chunk table, 3 x sscap
   int64_t sscap = 0;
   int nsub_s = 0;
@@ -252,18 +257,23 @@ struct gbn_plan_s {
   // (Re)allocates the per-bin arrays for the current geometry.
   void setup_bins() {
     free_bins();
-    stream_spread = stream_fit(g) ? 1 : 0;
+    tc = !spread_only && tc_fit(g);
+    stream_spread = tc || stream_fit(g) ? 1 : 0;
     const int last = g.dim - 1;
     ngrp = g.nb[0] * g.nb[1] * g.nb[2];
     ncol = ngrp / g.nb[last];
-    nbins = stream_spread ? ncol * g.nf[last] : ngrp;
+    nbins = stream_spread ? ncol * g.nkey[last] : ngrp;
+    sgrp_k = tc && g.dim == 2 ? g.bs[0] : g.nkey[last];
+    sgrp_n = stream_spread ? ncol * ((g.nkey[last] + sgrp_k - 1) / sgrp_k) : 0;
     const int64_t b0 = bytes;
     sb.bin_count = dev_alloc<int>(nbins, bytes, "bins");
     sb.bin_start = dev_alloc<int>(nbins, bytes, "bins");
-    sb.nsub_bin = dev_alloc<int>(nbins, bytes, "bins");
-    sb.sub_off = dev_alloc<int>(nbins, bytes, "bins");
+    if (!stream_spread) {
+      sb.nsub_bin = dev_alloc<int>(nbins, bytes, "bins");
+      sb.sub_off = dev_alloc<int>(nbins, bytes, "bins");
+    }
     sb.scan_scratch = dev_alloc<int>(scan_scratch_ints(nbins), bytes, "scan");
-    if (stream_spread) grp = dev_alloc<int>(4 * ((size_t)ngrp + ncol), bytes, "bin groups");
+    if (stream_spread) grp = dev_alloc<int>(4 * ((size_t)ngrp + sgrp_n), bytes, "bin groups");
     bin_bytes = bytes - b0;
   }
 
@@ -414,8 +424,24 @@ void gbn_plan_s::exec_fft(int batch, float2* data, int isign, cudaStream_t st, i
 
 namespace {
 
+// A word of page-locked host memory that a tensor-core kernel sets when a wait
+// runs out; looked at by every later call.  Allocated once, by the first plan
+// that uses such a kernel.
+int* tc_error_flag() {
+  static int* const flag = [] {
+    int* f = nullptr;
+    ck(cudaHostAlloc(reinterpret_cast<void**>(&f), sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped),
+       "error flag");
+    *f = 0;
+    return f;
+  }();
+  return flag;
+}
+
 void require_points(gbn_plan p) {
   if (!p) fail(GBN_ERR_ARG, "null plan");
+  if (p->tc && *reinterpret_cast<volatile int*>(tc_error_flag()))
+    fail(GBN_ERR_CUDA, "a tensor-core kernel gave up waiting; its results are not valid");
   if (p->M < 0) fail(GBN_ERR_STATE, "gbn_setpts has not been called on this plan");
 }
 
@@ -431,6 +457,11 @@ void run_spread(gbn_plan p, const SpreadArgs& a, cudaStream_t st) {
   // 2D: the streaming spreader for several transforms per call, the
   // warp-cooperative one (any sort order) for a single transform
   const bool stream = p->stream_spread && (a.g.dim == 3 || a.ntr >= 2);
+  if (stream && p->tc) {
+    ck(launch_spread_tc(a, tc_error_flag(), st), "spread kernel");
+    p->launches++;
+    return;
+  }
   ck(stream ? (a.g.dim == 2 ? launch_spread_stream2d(a, st) : launch_spread_stream3d(a, st))
             : (a.g.dim == 2 ? launch_spread2d(a, st) : launch_spread3d(a, st)),
      "spread kernel");
@@ -629,10 +660,22 @@ int gbn_plan_create(int dim, const int64_t* n_modes, double upsampfac, double ep
     g.inv_halfw = 2.0f / w;
     g.G = 1;
     g.Nimg = 1;
-    // 2D: 19-cell x bins (with w <= 7 the padded column is at most 26 rows,
+    // 2D: 19-cell x bins (with w <= 7 the padded column is at most 25 rows,
     // two overlapping 16-row halves of a warp in the streaming spreader)
     int binsz2[2] = {19, 32};
     int binsz3[3] = {8, 8, 8};
+    const char* sp = std::getenv("GBN_SPREAD");
+    const bool want_tc = sp && std::strcmp(sp, "mma") == 0;
+    // Plans of several transforms: the tiles of the tensor-core spreaders.
+    // Against the FP32 column spreaders: 3D 16 coils, 2.1 M samples 6.09 -> 3.7
+    // ms; 2D 131 072 samples, 16 transforms 148 -> 58 us, 64 transforms 401 ->
+    // 173 us a pass.  A plan of one transform keeps the FP32 kernels (the MMA's
+    // columns would be mostly empty).
+    if (!spread_only && w <= 7 && (want_tc || (!sp && ntrans >= 2))) {
+      binsz2[0] = tc_bin(2, w);
+      binsz3[0] = binsz3[1] = tc_bin(3, w);
+      binsz3[2] = 16;
+    }
     // tuning overrides: GBN_BINS2="b0,b1", GBN_BINS3="b0,b1,b2", GBN_INTERP_CG=1|2|4
     if (const char* e = std::getenv(dim == 2 ? "GBN_BINS2" : "GBN_BINS3")) {
       int v[3] = {0, 0, 0};
@@ -656,14 +699,15 @@ int gbn_plan_create(int dim, const int64_t* n_modes, double upsampfac, double ep
       int v = std::atoi(e);
       if (v == 64 || v == 128 || v == 256) g.interp_threads = v;
     }
-    if (const char* e = std::getenv("GBN_SPREAD"))
-      g.method_spread = std::strcmp(e, "gm") == 0       ? 1
-                        : std::strcmp(e, "wc") == 0     ? 2
-                        : std::strcmp(e, "stream") == 0 ? 3
-                        : std::strcmp(e, "rows") == 0   ? 4
-                        : std::strcmp(e, "quad") == 0   ? 5
-                        : std::strcmp(e, "mma") == 0    ? 6
-                                                        : 0;
+    if (sp)
+      g.method_spread = std::strcmp(sp, "gm") == 0       ? 1
+                        : std::strcmp(sp, "wc") == 0     ? 2
+                        : std::strcmp(sp, "stream") == 0 ? 3
+                        : std::strcmp(sp, "rows") == 0   ? 4
+                        : std::strcmp(sp, "quad") == 0   ? 5
+                        : want_tc                        ? 6
+                                                         : 0;
+    g.koff = (w / 2 + 1) & ~1;
     for (int d = 0; d < 3; ++d) {
       if (d < dim) {
         int64_t N = n_modes[d];
@@ -680,11 +724,12 @@ int gbn_plan_create(int dim, const int64_t* n_modes, double upsampfac, double ep
         int bs = dim == 2 ? binsz2[d] : binsz3[d];
         if (bs > nf) bs = (int)nf;
         g.bs[d] = bs;
-        g.nb[d] = (int)((nf + bs - 1) / bs);
-        g.pd[d] = bs + w;
+        g.nkey[d] = (int)nf + g.koff - w / 2;
+        g.nb[d] = (g.nkey[d] + bs - 1) / bs;
+        g.pd[d] = bs + w - 1;
         g.uscale[d] = (float)((double)nf / (2.0 * M_PI));
       } else {
-        g.n[d] = g.nf[d] = g.bs[d] = g.nb[d] = g.pd[d] = 1;
+        g.n[d] = g.nf[d] = g.bs[d] = g.nb[d] = g.pd[d] = g.nkey[d] = 1;
         g.uscale[d] = 0.f;
       }
       g.G *= g.nf[d];
@@ -724,6 +769,10 @@ int gbn_plan_create(int dim, const int64_t* n_modes, double upsampfac, double ep
     }
     p->fine = dev_alloc<float2>((size_t)ntrans * g.G, p->bytes, "fine grid");
     p->setup_bins();
+    if (p->tc) {
+      ck(tc_spread_prepare(), "spread kernel attributes");
+      tc_error_flag();
+    }
     p->sb.d_total = dev_alloc<int>(2, p->bytes, "scan");
     *out = p;
     return GBN_OK;
@@ -798,9 +847,10 @@ int gbn_setpts(gbn_plan p, int64_t M, const float* k0, const float* k1, const fl
     }();
     int64_t subcap = M / maxsub_i + (M < p->ngrp ? M : p->ngrp) + 1;
     // spread chunks of the streaming kernel: one CTA batch at most
-    const int chunk = p->g.dim == 2 ? kStreamChunk2 : kStreamChunk;
+    const int chunk = p->tc ? (p->g.dim == 2 ? kTcChunk2 : kTcChunk3)
+                            : (p->g.dim == 2 ? kStreamChunk2 : kStreamChunk);
     const int maxsub_s = maxsub < chunk ? maxsub : chunk;
-    int64_t sscap = p->stream_spread ? M / maxsub_s + (M < p->ncol ? M : p->ncol) + 1 : 0;
+    int64_t sscap = p->stream_spread ? M / maxsub_s + (M < p->sgrp_n ? M : p->sgrp_n) + 1 : 0;
     if (M > p->Mcap || subcap > p->subcap || sscap > p->sscap) {
       // free the previous point buffers before the new ones (bytes tally)
       int64_t cap = M > p->Mcap ? M : p->Mcap;
@@ -833,18 +883,19 @@ int gbn_setpts(gbn_plan p, int64_t M, const float* k0, const float* k1, const fl
       const int last = g.dim - 1;
       Geom gs = g;  // sort key: the bins of the other axes, then the last-axis cell
       gs.bs[last] = 1;
-      gs.nb[last] = g.nf[last];
+      gs.nb[last] = g.nkey[last];
       ck(sort_points(gs, M, k, maxsub, p->sb, st, false), "sort");
       int* q = p->grp;
       GroupBuffers gi{q, q + p->ngrp, q + 2 * p->ngrp, q + 3 * p->ngrp,
                       p->sb.sub_bin, p->sb.sub_start, p->sb.sub_count};
       q += 4 * (size_t)p->ngrp;
-      GroupBuffers gc{q, q + p->ncol, q + 2 * p->ncol, q + 3 * p->ncol,
+      const int ns = p->sgrp_n;
+      GroupBuffers gc{q, q + ns, q + 2 * (size_t)ns, q + 3 * (size_t)ns,
                       p->ssub, p->ssub + p->sscap, p->ssub + 2 * p->sscap};
-      ck(build_group_table(p->ngrp, g.nb[last], g.bs[last], g.nf[last], maxsub_i, p->sb, gi,
+      ck(build_group_table(p->ngrp, g.nb[last], g.bs[last], g.nkey[last], maxsub_i, p->sb, gi,
                            p->sb.d_total, st),
          "interp groups");
-      ck(build_group_table(p->ncol, 1, g.nf[last], g.nf[last], maxsub_s, p->sb, gc,
+      ck(build_group_table(ns, ns / p->ncol, p->sgrp_k, g.nkey[last], maxsub_s, p->sb, gc,
                            p->sb.d_total + 1, st),
          "spread chunks");
     } else {
@@ -1070,13 +1121,17 @@ int gbn_plan_tune(gbn_plan p, const int* bins, int interp_method, int maxsub_cap
       for (int d = 0; d < g.dim; ++d) {
         if (bins[d] < 1 || bins[d] > 64) fail(GBN_ERR_ARG, "bin sizes must be in [1, 64]");
         t.bs[d] = bins[d] > g.nf[d] ? g.nf[d] : bins[d];
-        t.nb[d] = (g.nf[d] + t.bs[d] - 1) / t.bs[d];
-        t.pd[d] = t.bs[d] + g.w;
+        t.nb[d] = (g.nkey[d] + t.bs[d] - 1) / t.bs[d];
+        t.pd[d] = t.bs[d] + g.w - 1;
       }
       t.tile = t.pd[0] * t.pd[1] * t.pd[2];
       if ((int64_t)t.tile * 8 > kTileSmemBudget) fail(GBN_ERR_ARG, "tile does not fit shared memory");
       g = t;
       p->setup_bins();
+      if (p->tc) {
+        ck(tc_spread_prepare(), "spread kernel attributes");
+        tc_error_flag();
+      }
       p->M = -1;  // points must be set again
     }
     if (interp_method >= 0) {

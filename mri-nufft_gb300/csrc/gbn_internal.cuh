@@ -27,7 +27,9 @@ struct Geom {
   int nf[3];     // fine grid per axis (unused axes = 1)
   int bs[3];     // bin size per axis (unused axes = 1)
   int nb[3];     // number of bins per axis
-  int pd[3];     // padded tile extent per axis = bs + w (unused axes = 1)
+  int pd[3];     // padded tile extent per axis = bs + w - 1 (unused axes = 1)
+  int nkey[3];   // sort keys per axis: a sample's key is its first footprint cell + koff
+  int koff;      // floor(w / 2) rounded up to even, so that even-sized bins start on even cells
   int w;         // kernel width in cells
   float beta;    // ES shape parameter
   float halfw;   // w / 2
@@ -42,8 +44,7 @@ struct Geom {
                       // 5: 3D tile warp-cooperative, 6: tiles
   int method_spread;  // 0: automatic, 1: global atomics, 2: warp-cooperative atomics,
                       // 3: 3D column streaming, 4: 3D bin-tile rows,
-                      // 5: 3D quadrant streaming (8 x 8 bins),
-                      // 6: 3D quadrant tiles on the tensor cores (8 x 8 bins, w = 7)
+                      // 5: 3D quadrant streaming (8 x 8 bins), 6: tensor cores (tc_bins)
   int interp_threads; // CTA size of the tile interp kernel (0: 128)
   int spread_cg;      // coils per pass of the streaming spreader (0: automatic)
   int quad_minb;      // resident CTAs per SM of the 4-coil quadrant spreader (0: 3)
@@ -141,10 +142,18 @@ __device__ __forceinline__ float fold_coord(float k, float uscale, int nf) {
   return u;
 }
 
-__device__ __forceinline__ int cell_of(float u, int nf) {
-  int f = (int)floorf(u);
-  f = f < 0 ? 0 : f;
-  return f > nf - 1 ? nf - 1 : f;
+// Sort key of a folded coordinate, the first footprint cell + koff in
+// [0, nkey).  Samples whose footprint starts at nf - floor(w / 2) or later
+// move one period down (u in [-1, 0), an exact subtraction), so that every
+// footprint starts in [-floor(w / 2), nf - floor(w / 2)).
+__device__ __forceinline__ int key_of(float& u, int nf, const Geom& g, int d) {
+  int o = (int)ceilf(u - g.halfw);
+  if (o + (g.w >> 1) >= nf) {
+    u -= (float)nf;
+    o = (int)ceilf(u - g.halfw);
+  }
+  const int k = o + g.koff;
+  return k < 0 ? 0 : k > g.nkey[d] - 1 ? g.nkey[d] - 1 : k;
 }
 
 // Kernel width and shape from the published exponential-of-semicircle rules
@@ -223,5 +232,24 @@ inline bool stream_fit(const Geom& g) {
 // Samples per chunk of the column-streaming spreaders (3D, 2D).
 constexpr int kStreamChunk = 512;
 constexpr int kStreamChunk2 = 256;
+
+// Tensor-core spreaders (gbn_tc_spread.cu): bins of the leading axes such that
+// the footprints of a bin's origins span 16 cells (2D, kept even so that tiles
+// start on 16-byte boundaries) or 11 (3D: 121 of the 128 rows of an MMA), and
+// the samples of one chunk (2D: all strengths of a chunk stay in registers).
+inline int tc_bin(int dim, int w) { return dim == 2 ? (17 - w) & ~1 : 12 - w; }
+inline bool tc_fit(const Geom& g) {
+  if (g.w > 7 || !(g.method_spread == 0 || g.method_spread == 6)) return false;
+  const int b = tc_bin(g.dim, g.w);
+  for (int d = 0; d < g.dim; ++d)
+    if ((d < g.dim - 1 && g.bs[d] != b) || g.nf[d] % 2 || g.nf[d] > 16000) return false;
+  return true;
+}
+constexpr int kTcChunk2 = 128;
+constexpr int kTcChunk3 = 512;
+cudaError_t tc_spread_prepare();
+// a.s is the table of tile chunks (2D) or column chunks (3D); *err is set if a
+// wait runs out
+cudaError_t launch_spread_tc(const SpreadArgs& a, int* err, cudaStream_t st);
 
 }  // namespace gbn

@@ -2,7 +2,7 @@
 // interpolation kernels over bin-sorted samples.
 //
 // One CTA handles one subproblem: up to `maxsub` samples of one bin.  The
-// padded fine-grid tile of the bin (bin extent + w cells per axis, with
+// padded fine-grid tile of the bin (bin extent + w - 1 cells per axis, with
 // periodic wrap) is staged in shared memory for `CG` transforms (coils) at a
 // time.  Kernel weights are evaluated once per sample and axis per coil pass
 // and reused by every coil of the pass.
@@ -69,7 +69,7 @@ __device__ __forceinline__ void bin_origin(const Geom& g, int b, int* o) {
   for (int d = DIM - 1; d >= 0; --d) {
     int bd = r % g.nb[d];
     r /= g.nb[d];
-    o[d] = bd * g.bs[d] - (g.w >> 1);
+    o[d] = bd * g.bs[d] - g.koff;
   }
 }
 
@@ -1022,14 +1022,14 @@ spread_rows3d_kernel(SpreadArgs a) {
 // ---------------------------------------------------------------------------
 // Spreading, 3D column-streaming kernel (widths w <= 7).
 //
-// With the sort keyed on (x bin, y bin, z cell), the samples of one column
+// With the sort keyed on (x bin, y bin, first z cell), the samples of one column
 // of bins (bs0 x bs1 cells across, the whole z extent) arrive in z order.  A
 // CTA takes a chunk of <= kStreamBatch consecutive samples of one column.
 // Thread t owns row (i0, i1) of the column's padded (bs0 + w) x (bs1 + w)
 // cross-section (two i0 rows per warp, as in the row kernel) and keeps a
-// window of 8 z cells in registers: cell z lives in slot z & 7.  A sample in
-// z cell f covers cells [f - w/2, f - w/2 + 7], so the window is anchored at
-// zb = f - floor(w/2); when the samples reach a later anchor, the slots whose
+// window of 8 z cells in registers: cell z lives in slot z & 7.  A sample
+// covers its first cell and the w - 1 after it, so the window is anchored at
+// that cell; when the samples reach a later anchor, the slots whose
 // cells fall out of the window are added to the fine grid (float2 global
 // atomics) and cleared.  Each sample's z weights are staged already rotated
 // into slot order, so the accumulation indexes registers statically.
@@ -1109,9 +1109,8 @@ spread_stream3d_kernel(SpreadArgs a) {
   const int p0 = a.s.sub_start[sub];
   const int cnt = imin(a.s.sub_count[sub], kStreamBatch);
   const int w = W > 0 ? W : g.w;
-  const int hw = w >> 1;
-  const int o0 = (col / g.nb[1]) * g.bs[0] - hw;
-  const int o1 = (col % g.nb[1]) * g.bs[1] - hw;
+  const int o0 = (col / g.nb[1]) * g.bs[0] - g.koff;
+  const int o1 = (col % g.nb[1]) * g.bs[1] - g.koff;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // warp w owns rows i0 = 2w, 2w+1 (16 lanes each along i1)
   const int i0 = 2 * warp + (lane >> 4);
@@ -1132,18 +1131,9 @@ spread_stream3d_kernel(SpreadArgs a) {
     const int a1 = weights_rt<W>(a.s.u[1][pos], g, wt) - o1;  // 0 .. bs1
 #pragma unroll
     for (int k = 0; k < 8; ++k) s_w1[t * 8 + k] = k < w ? wt[k] : 0.f;
-    const float u2 = a.s.u[2][pos];
-    const int zs = cell_of(u2, nf2) - hw;
-    const int off = weights_rt<W>(u2, g, wt) - zs;  // 0 or 1
+    const int zs = weights_rt<W>(a.s.u[2][pos], g, wt);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const int m = k - off;
-      float v = 0.f;
-#pragma unroll
-      for (int kk = 0; kk < WidthTraits<W>::WM; ++kk)
-        if (kk == m && kk < w) v = wt[kk];
-      s_w2[t * 8 + ((zs + k) & 7)] = v;
-    }
+    for (int k = 0; k < 8; ++k) s_w2[t * 8 + ((zs + k) & 7)] = k < w ? wt[k] : 0.f;
     unsigned wm = 0;
 #pragma unroll
     for (int q = 0; q < GBN_THREADS / 32; ++q)
@@ -1294,10 +1284,9 @@ spread_quad3d_kernel(SpreadArgs a) {
   const int p0 = a.s.sub_start[sub];
   const int cnt = imin(a.s.sub_count[sub], kStreamBatch);
   const int w = W > 0 ? W : g.w;
-  const int hw = w >> 1;
   const int qx = (blockIdx.x >> 1) & 1, qy = blockIdx.x & 1;
-  const int b0 = (col / g.nb[1]) * g.bs[0] - hw;  // column origin (footprint frame)
-  const int b1 = (col % g.nb[1]) * g.bs[1] - hw;
+  const int b0 = (col / g.nb[1]) * g.bs[0] - g.koff;  // column origin (footprint frame)
+  const int b1 = (col % g.nb[1]) * g.bs[1] - g.koff;
   const int o0 = b0 + 4 * qx, o1 = b1 + 4 * qy;   // quadrant origin
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int pdq = 4 + w;
@@ -1342,18 +1331,9 @@ spread_quad3d_kernel(SpreadArgs a) {
       const int a1 = weights_rt<W>(a.s.u[1][pos], g, wt) - o1;
 #pragma unroll
       for (int k = 0; k < 8; ++k) s_w1[t * 8 + k] = k < w ? wt[k] : 0.f;
-      const float u2 = a.s.u[2][pos];
-      const int zs = cell_of(u2, nf2) - hw;
-      const int off = weights_rt<W>(u2, g, wt) - zs;  // 0 or 1
+      const int zs = weights_rt<W>(a.s.u[2][pos], g, wt);
 #pragma unroll
-      for (int k = 0; k < 8; ++k) {
-        const int m = k - off;
-        float v = 0.f;
-#pragma unroll
-        for (int kk = 0; kk < WidthTraits<W>::WM; ++kk)
-          if (kk == m && kk < w) v = wt[kk];
-        s_w2[t * 8 + ((zs + k) & 7)] = v;
-      }
+      for (int k = 0; k < 8; ++k) s_w2[t * 8 + ((zs + k) & 7)] = k < w ? wt[k] : 0.f;
       // warp q's threads own quadrant rows (32 q) / pdq .. (32 q + 31) / pdq along x
       unsigned wm = 0;
 #pragma unroll
@@ -1445,14 +1425,14 @@ spread_quad3d_kernel(SpreadArgs a) {
 // ---------------------------------------------------------------------------
 // Spreading, 2D column-streaming kernel (widths w <= 7).
 //
-// The sort is keyed on (x bin, y cell) with bs0 + w <= 32, so the samples of
+// The sort is keyed on (x bin, first y cell) with bs0 + w <= 33, so the samples of
 // one column (bs0 cells along x, the whole y extent) arrive in y order.  A
 // CTA takes a chunk of <= kStream2Batch consecutive samples of one column;
 // lane l of every warp owns row i0 = l of the column's padded cross-section
 // (32 rows along x) and keeps an 8-cell window along y in registers (cell y
 // in slot y & 7), for the CG transforms of its warp; the CTA's warps cover
-// different transforms of the same staged samples.  Samples in y cell f
-// cover cells [f - w/2, f - w/2 + 7]; when the anchor moves, the slots that
+// different transforms of the same staged samples.  The window is anchored at
+// the samples' first cell; when the anchor moves, the slots that
 // leave the window are added to the fine grid with float2 atomics.  The
 // kernel weights are evaluated once per chunk for every transform.
 // ---------------------------------------------------------------------------
@@ -1481,8 +1461,7 @@ spread_stream2d_kernel(SpreadArgs a) {
   const int p0 = a.s.sub_start[sub];
   const int cnt = imin(a.s.sub_count[sub], kStream2Batch);
   const int w = W > 0 ? W : g.w;
-  const int hw = w >> 1;
-  const int o0 = col * g.bs[0] - hw;
+  const int o0 = col * g.bs[0] - g.koff;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const bool own = lane < g.pd[0];
   const int nf1 = g.nf[1];
@@ -1496,18 +1475,9 @@ spread_stream2d_kernel(SpreadArgs a) {
     const int a0 = weights_rt<W>(a.s.u[0][pos], g, wt) - o0;  // 0 .. bs0
 #pragma unroll
     for (int k = 0; k < 8; ++k) s_w0[t * 8 + k] = k < w ? wt[k] : 0.f;
-    const float u1 = a.s.u[1][pos];
-    const int zs = cell_of(u1, nf1) - hw;
-    const int off = weights_rt<W>(u1, g, wt) - zs;  // 0 or 1
+    const int zs = weights_rt<W>(a.s.u[1][pos], g, wt);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const int m = k - off;
-      float v = 0.f;
-#pragma unroll
-      for (int kk = 0; kk < WidthTraits<W>::WM; ++kk)
-        if (kk == m && kk < w) v = wt[kk];
-      s_w1[t * 8 + ((zs + k) & 7)] = v;
-    }
+    for (int k = 0; k < 8; ++k) s_w1[t * 8 + ((zs + k) & 7)] = k < w ? wt[k] : 0.f;
     s_hd[t] = (unsigned)(zs + 8) | ((unsigned)a0 << 14);
   }
 
@@ -1600,9 +1570,8 @@ spread_half2d_kernel(SpreadArgs a) {
   const int p0 = a.s.sub_start[sub];
   const int cnt = imin(a.s.sub_count[sub], kStream2Batch);
   const int w = W > 0 ? W : g.w;
-  const int hw = w >> 1;
   const int S = 17 - w;  // first footprint origin of half 1
-  const int o0 = col * g.bs[0] - hw;
+  const int o0 = col * g.bs[0] - g.koff;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int half = lane >> 4;
   const int row = (lane & 15) + (half ? S : 0);
@@ -1618,18 +1587,9 @@ spread_half2d_kernel(SpreadArgs a) {
     const int a0 = weights_rt<W>(a.s.u[0][pos], g, wt) - o0;  // 0 .. bs0
 #pragma unroll
     for (int k = 0; k < 8; ++k) s_w0[t * 8 + k] = k < w ? wt[k] : 0.f;
-    const float u1 = a.s.u[1][pos];
-    const int zs = cell_of(u1, nf1) - hw;
-    const int off = weights_rt<W>(u1, g, wt) - zs;  // 0 or 1
+    const int zs = weights_rt<W>(a.s.u[1][pos], g, wt);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const int m = k - off;
-      float v = 0.f;
-#pragma unroll
-      for (int kk = 0; kk < WidthTraits<W>::WM; ++kk)
-        if (kk == m && kk < w) v = wt[kk];
-      s_w1[t * 8 + ((zs + k) & 7)] = v;
-    }
+    for (int k = 0; k < 8; ++k) s_w1[t * 8 + ((zs + k) & 7)] = k < w ? wt[k] : 0.f;
     s_hd[t] = (unsigned)(zs + 8) | ((unsigned)a0 << 14);
   }
   __syncthreads();
@@ -2029,20 +1989,12 @@ cudaError_t launch_spread_quad_t(const SpreadArgs& a, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-}  // namespace gbn
-
-#include "gbn_mma_spread.cuh"
-
-namespace gbn {
-
 // a.s is the column-chunk table (sub_bin = column index)
 inline cudaError_t dispatch_spread_stream3d(const SpreadArgs& a, cudaStream_t st) {
   int cg = a.ntr >= 3 ? 4 : a.ntr;
   if (a.g.spread_cg == 1 || a.g.spread_cg == 2 || a.g.spread_cg == 4) cg = imin(cg, a.g.spread_cg);
   // 8 x 8 bins: quadrant CTAs (measured 7 % faster than whole columns on the
   // 3D kooshball); GBN_SPREAD=stream keeps the column kernel
-  if (a.g.method_spread == 6 && a.g.w == 7 && a.g.bs[0] == 8 && a.g.bs[1] == 8)
-    return launch_spread_mma3d(a, st);
   if ((a.g.method_spread == 0 || a.g.method_spread == 5) && a.g.bs[0] == 8 && a.g.bs[1] == 8) {
     if (a.g.w == 7) {
       // 4 coils per pass at 3 CTAs per SM (170 registers, no spills;

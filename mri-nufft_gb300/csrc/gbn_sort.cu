@@ -1,7 +1,8 @@
 // Bin sort of the non-uniform points (the "setpts" step).
 //
 // A counting sort over spatial bins of the fine grid:
-//   1. each sample is folded to fine-grid units, assigned its bin and a rank
+//   1. each sample is folded to fine-grid units, assigned the bin of its first
+//      footprint cell and a rank
 //      inside the bin with a warp-aggregated atomic (lanes of one warp that
 //      share a bin receive consecutive ranks in lane order, so runs of
 //      consecutive input samples stay contiguous after the sort and the
@@ -26,8 +27,7 @@ __global__ void bin_count_kernel(Geom g, int64_t M, const float* __restrict__ k0
   int b = 0;
   for (int d = 0; d < g.dim; ++d) {
     float u = fold_coord(ks[d][j], g.uscale[d], g.nf[d]);
-    int f = cell_of(u, g.nf[d]);
-    b = b * g.nb[d] + f / g.bs[d];
+    b = b * g.nb[d] + key_of(u, g.nf[d], g, d) / g.bs[d];
   }
   const int lane = threadIdx.x & 31;
   unsigned peers = __match_any_sync(active, b);
@@ -49,9 +49,13 @@ __global__ void scatter_kernel(Geom g, int64_t M, const float* __restrict__ k0,
   if (j >= M) return;
   int pos = bin_start[bin_of[j]] + rank_of[j];
   perm[pos] = (int)j;
-  u0[pos] = fold_coord(k0[j], g.uscale[0], g.nf[0]);
-  u1[pos] = fold_coord(k1[j], g.uscale[1], g.nf[1]);
-  if (g.dim == 3) u2[pos] = fold_coord(k2[j], g.uscale[2], g.nf[2]);
+  const float* ks[3] = {k0, k1, k2};
+  float* us[3] = {u0, u1, u2};
+  for (int d = 0; d < g.dim; ++d) {
+    float u = fold_coord(ks[d][j], g.uscale[d], g.nf[d]);
+    key_of(u, g.nf[d], g, d);
+    us[d][pos] = u;
+  }
 }
 
 __global__ void nsub_kernel(int nbins, const int* __restrict__ bin_count, int maxsub,
