@@ -160,6 +160,7 @@ struct gbn_plan_s {
   float* dec[3] = {nullptr, nullptr, nullptr};
   float2* fine = nullptr;
   float2* kbuf = nullptr;  // ntrans x M residual scratch for dc
+  unsigned* fmax = nullptr;  // ntrans: largest fine cell of each transform (2D tensor-core interp)
   int64_t kbuf_cap = 0;
 
   // sort state
@@ -235,6 +236,7 @@ struct gbn_plan_s {
     for (int d = 0; d < 3; ++d) dev_free(dec[d]);
     dev_free(fine);
     dev_free(kbuf);
+    dev_free(fmax);
     dev_free(tw256);
     dev_free(tw512);
     free_points();
@@ -438,6 +440,15 @@ int* tc_error_flag() {
   return flag;
 }
 
+// what a plan with tensor-core tables needs beyond them
+void setup_tc(gbn_plan p) {
+  if (!p->tc) return;
+  ck(tc_spread_prepare(), "spread kernel attributes");
+  ck(tc_interp_prepare(), "interp kernel attributes");
+  tc_error_flag();
+  if (!p->fmax && p->fft512) p->fmax = dev_alloc<unsigned>(p->ntrans, p->bytes, "fine-grid maxima");
+}
+
 void require_points(gbn_plan p) {
   if (!p) fail(GBN_ERR_ARG, "null plan");
   if (p->tc && *reinterpret_cast<volatile int*>(tc_error_flag()))
@@ -445,9 +456,23 @@ void require_points(gbn_plan p) {
   if (p->M < 0) fail(GBN_ERR_STATE, "gbn_setpts has not been called on this plan");
 }
 
+// Tensor-core interpolation: 2D plans with its tables whose transforms leave the
+// largest fine cell, from 25 transforms on.  Radial 256 x 512 samples, 512^2 grids,
+// interp + transforms against the gather kernel: 64 transforms 320 / 457 us, 32
+// 198 / 235, 24 173 / 185 (spiral 176 / 176), 16 136 / 131.
+bool use_tc_interp(gbn_plan p, int ntr) { return p->tc && p->fft512 && p->g.method_interp == 0 && ntr > 24; }
+
 void run_interp(gbn_plan p, const InterpArgs& a, cudaStream_t st) {
   if (a.s.nsub == 0) return;
   Span span(p, GBN_STAGE_INTERP, st);
+  if (use_tc_interp(p, a.ntr)) {
+    InterpArgs t = a;
+    t.s = p->sorted_spread();
+    t.fmax = p->fmax;
+    ck(launch_interp_tc(t, tc_error_flag(), st), "interp kernel");
+    p->launches++;
+    return;
+  }
   ck(a.g.dim == 2 ? launch_interp2d(a, st) : launch_interp3d(a, st), "interp kernel");
   p->launches++;
 }
@@ -477,8 +502,11 @@ void run_crop(gbn_plan p, const CropArgs& a, cudaStream_t st) {
   ck(launch_crop(a, st), "crop pass");
   p->launches++;
 }
-// op: pad + forward transform (fused line transforms on 256^3 grids)
-void run_pad_fft(gbn_plan p, const PadArgs& a, int isign, cudaStream_t st) {
+// op: pad + forward transform (fused line transforms on 256^3 and 512^2 grids);
+// before an interpolation that scales by it, also the largest cell of every grid
+void run_pad_fft(gbn_plan p, const PadArgs& pa, int isign, cudaStream_t st, bool interp_next = false) {
+  PadArgs a = pa;
+  a.fmax = interp_next && use_tc_interp(p, a.ntr) ? p->fmax : nullptr;
   if (p->fft512) {
     Span span(p, GBN_STAGE_FFT, st);
     ck(launch_fft512_op(a, p->tw512, isign, st), "fused pad + transform");
@@ -769,10 +797,7 @@ int gbn_plan_create(int dim, const int64_t* n_modes, double upsampfac, double ep
     }
     p->fine = dev_alloc<float2>((size_t)ntrans * g.G, p->bytes, "fine grid");
     p->setup_bins();
-    if (p->tc) {
-      ck(tc_spread_prepare(), "spread kernel attributes");
-      tc_error_flag();
-    }
+    setup_tc(p);
     p->sb.d_total = dev_alloc<int>(2, p->bytes, "scan");
     *out = p;
     return GBN_OK;
@@ -937,7 +962,7 @@ int gbn_op(gbn_plan p, const void* img, const void* smaps, void* ksp, int B, int
     for_each_pass(p, s != nullptr, B, C, [&](int b, int c0, int T) {
       PadArgs pa = s ? pad_args(p, x + (int64_t)b * g.Nimg, s + (int64_t)c0 * g.Nimg, T, 0)
                      : pad_args(p, x + (int64_t)c0 * g.Nimg, nullptr, T, 0);
-      run_pad_fft(p, pa, isign, st);
+      run_pad_fft(p, pa, isign, st, true);
       int64_t row = s ? (int64_t)b * C + c0 : c0;
       run_interp(p, interp_args(p, p->fine, y + row * p->M, T, scale, INTERP_STORE), st);
     });
@@ -1002,7 +1027,7 @@ int gbn_dc(gbn_plan p, const void* img, const void* obs, const float* density,
     for_each_pass(p, s != nullptr, B, C, [&](int b, int c0, int T) {
       PadArgs pa = s ? pad_args(p, x + (int64_t)b * g.Nimg, s + (int64_t)c0 * g.Nimg, T, 0)
                      : pad_args(p, x + (int64_t)c0 * g.Nimg, nullptr, T, 0);
-      run_pad_fft(p, pa, -1, st);
+      run_pad_fft(p, pa, -1, st, true);
       int64_t row = s ? (int64_t)b * C + c0 : c0;
       InterpArgs ia = interp_args(p, p->fine, p->kbuf, T, scale, INTERP_RESID);
       ia.obs = yo + row * p->M;
@@ -1128,10 +1153,7 @@ int gbn_plan_tune(gbn_plan p, const int* bins, int interp_method, int maxsub_cap
       if ((int64_t)t.tile * 8 > kTileSmemBudget) fail(GBN_ERR_ARG, "tile does not fit shared memory");
       g = t;
       p->setup_bins();
-      if (p->tc) {
-        ck(tc_spread_prepare(), "spread kernel attributes");
-        tc_error_flag();
-      }
+      setup_tc(p);
       p->M = -1;  // points must be set again
     }
     if (interp_method >= 0) {

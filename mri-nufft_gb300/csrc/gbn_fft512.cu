@@ -45,6 +45,7 @@
 #include <vector>
 
 #include "gbn_dft.cuh"
+#include "gbn_tc.cuh"
 
 namespace gbn {
 
@@ -151,6 +152,7 @@ f512_pad_y_kernel(PadArgs a, const float2* __restrict__ tw, int conj) {
   const float2* sm = a.smaps ? a.smaps + (int64_t)c * g.Nimg : nullptr;
   float f0 = a.scale;
   if (a.dec[0]) f0 *= a.dec[0][valid ? ix : 0];
+  if (a.fmax && blockIdx.x == 0 && threadIdx.x == 0) a.fmax[c] = 0;  // the x pass comes after
   float2 x[32];
 #pragma unroll
   for (int q = 0; q < 32; ++q) {
@@ -198,6 +200,7 @@ struct F512Lines {
   int64_t G;
   int n_axis;     // image size along x
   int conj;
+  unsigned* fmax;  // null, or the largest |re|, |im| written for each transform
   const float2* tw;
 };
 
@@ -227,6 +230,7 @@ __global__ void __launch_bounds__(kT, 2) f512_x_kernel(F512Lines a) {
 #pragma unroll
   for (int k1 = 0; k1 < 32; ++k1) s_x[(k1 * 16 + b) * kL + l] = f2mul(x[k1], s_tw[k1 * 16 + b]);
   __syncthreads();
+  float mx = 0.f;
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     const int k1 = b + 16 * h;
@@ -239,8 +243,15 @@ __global__ void __launch_bounds__(kT, 2) f512_x_kernel(F512Lines a) {
       if (out_on<OUT>(k1, k2, a.n_axis)) {
         const float2 v = w[pos16(k2)];
         base[(k1 + 32 * k2) * kN] = a.conj ? f2conj(v) : v;
+        if (OUT == kAll) mx = fmaxf(mx, fmaxf(tc::finite_abs(v.x), tc::finite_abs(v.y)));
       }
     }
+  }
+  if (OUT == kAll && a.fmax) {
+    // the atomic only where this warp raises the maximum
+    const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(mx));
+    unsigned* const p = a.fmax + blockIdx.y;
+    if ((threadIdx.x & 31) == 0 && m > *reinterpret_cast<volatile unsigned*>(p)) atomicMax(p, m);
   }
 }
 
@@ -414,7 +425,8 @@ cudaError_t launch_fft512_op(const PadArgs& pa, const float2* tw, int isign, cud
   const dim3 gy((g.n[0] + kL - 1) / kL, pa.ntr);
   if (g.n[1] == 256) f512_pad_y_kernel<kHalf><<<gy, kT, kYSmem, st>>>(pa, tw, conj);
   else f512_pad_y_kernel<kModes><<<gy, kT, kYSmem, st>>>(pa, tw, conj);
-  const F512Lines x = x_lines(pa.fine, g, tw, conj);
+  F512Lines x = x_lines(pa.fine, g, tw, conj);
+  x.fmax = pa.fmax;
   const dim3 gx(kN / kL, pa.ntr);
   if (g.n[0] == 256) f512_x_kernel<kHalf, kAll><<<gx, kT, kXSmem, st>>>(x);
   else f512_x_kernel<kModes, kAll><<<gx, kT, kXSmem, st>>>(x);

@@ -77,6 +77,7 @@ struct InterpArgs {
   float2* out;          // ntr x M (original sample order)
   const float2* obs;    // INTERP_RESID: ntr x M
   const float* density; // optional, M
+  const unsigned* fmax; // tensor-core kernel: bits of the largest |re|, |im| of each fine grid
   int ntr;              // transforms in this launch
   float scale;
   int mode;
@@ -248,6 +249,9 @@ inline bool tc_fit(const Geom& g) {
 constexpr int kTcChunk2 = 128;
 constexpr int kTcChunk3 = 512;
 cudaError_t tc_spread_prepare();
+cudaError_t tc_interp_prepare();
+// 2D; a.s is the table of tile chunks, a.fmax left by the fused transforms
+cudaError_t launch_interp_tc(const InterpArgs& a, int* err, cudaStream_t st);
 // a.s is the table of tile chunks (2D) or column chunks (3D); *err is set if a
 // wait runs out
 cudaError_t launch_spread_tc(const SpreadArgs& a, int* err, cudaStream_t st);

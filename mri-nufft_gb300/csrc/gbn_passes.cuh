@@ -11,6 +11,7 @@ struct PadArgs {
   const float2* smaps;  // SENSE: ntr coil maps (null: calibrationless)
   const float* dec[3];  // 1/phihat per axis, indexed by image array index (null: 1)
   float2* fine;         // ntr fine grids (every cell written)
+  unsigned* fmax;       // null, or where the transform leaves the bits of each grid's largest |re|, |im|
   int ntr;
   int conj_in;          // use conj(img) and conj(smaps)
   float scale;

@@ -2,14 +2,17 @@
 // accumulators in tensor memory), mbarriers, the split of fp32 values into
 // two fp16 parts, vector reductions.
 //
-// Operands lie in shared memory as K-major core matrices without swizzle: 8
-// rows (of M or N) x 16 bytes (8 samples), 128 contiguous bytes.  The core
-// matrix of row group r and sample octet o sits at r * 128 + o * lbo.
+// Operands lie in shared memory as core matrices of 128 contiguous bytes without
+// swizzle: K-major, 8 rows (of M or N) x 8 k values of 16 bytes a row; MN-major,
+// 8 k x 8 rows.  The core matrix of row octet r and k octet o sits at
+// r * 128 + o * lbo.
 #pragma once
 
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include "gbn_internal.cuh"
 
 namespace gbn {
 namespace tc {
@@ -69,6 +72,9 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo) {
   return (uint64_t)((addr >> 4) & 0x3fff) | (uint64_t)((lbo >> 4) & 0x3fff) << 16 |
          (uint64_t)(128 >> 4) << 32 | (uint64_t)1 << 46;
 }
+// instruction descriptor bit: A is MN-major, its core matrices 8 k x 8 rows with
+// the rows contiguous
+constexpr uint32_t kMajorA = 1u << 15;
 // instruction descriptor: M = 128, fp16 A and B, fp32 D
 __host__ __device__ constexpr uint32_t idesc_f16(uint32_t n) {
   return (1u << 4) | ((n >> 3) << 17) | ((128u >> 4) << 24);
@@ -109,6 +115,15 @@ __device__ __forceinline__ void tmem_ld8(uint32_t addr, float (&v)[8]) {
                : "memory");
 #pragma unroll
   for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
+}
+__device__ __forceinline__ void tmem_ld4(uint32_t addr, float (&v)[4]) {
+  uint32_t r[4];
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+#pragma unroll
+  for (int i = 0; i < 4; ++i) v[i] = __uint_as_float(r[i]);
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_zero16(uint32_t addr) {
@@ -156,6 +171,136 @@ __device__ __forceinline__ float finite_abs(float v) {  // 0 for infinities and 
   return m <= 3.402823466e38f ? m : 0.f;
 }
 __device__ __forceinline__ float pow2(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }
+
+// scales of the split factors: x weights 2^8, y and z weights 2^7, strengths
+// 2^(6 - e), fine cells 2^(14 - e) with 2^e the largest of them
+constexpr float kScaleX = 256.0f, kScaleY = 128.0f, kScaleC = 64.0f;
+// mean relative loss of an accumulator for each step that truncates it, given
+// back with the cross terms
+constexpr float kTrunc = 6e-8f;
+constexpr int kTcRows = 11;   // 3D cross-section rows per axis
+constexpr int kRound = 128;   // largest round of samples (3D)
+
+// the w <= 7 kernel weights t0 .. t0 + N - 1 of coordinate u; returns the first cell
+template <int N>
+__device__ __forceinline__ int weights_part(float u, const Geom& g, int t0, float (&wt)[N]) {
+  const int i0 = (int)ceilf(u - g.halfw);
+  const float x0 = (float)i0 - u;
+#pragma unroll
+  for (int t = 0; t < N; ++t)
+    wt[t] = t0 + t < g.w ? es_eval(x0 + (float)(t0 + t), g.beta, g.inv_halfw) : 0.f;
+  return i0;
+}
+
+__device__ __forceinline__ int wrap_once(int i, int n) {
+  const int m = i < 0 ? i + n : (i >= n ? i - n : i);
+  return (unsigned)m < (unsigned)n ? m : wrap_idx(i, n);
+}
+
+// v = hi + lo, stored as halves `lo_off` bytes apart
+__device__ __forceinline__ void put_split(unsigned char* p, int lo_off, float v) {
+  const __half h = __float2half_rn(v);
+  *reinterpret_cast<__half*>(p) = h;
+  *reinterpret_cast<__half*>(p + lo_off) = __float2half_rn(v - __half2float(h));
+}
+
+// the split product of two split factors, 8 samples: h = xh yh rounded,
+// l = (xh yh - h) + xh yl + xl yh, whose first term is exact
+__device__ __forceinline__ void mul_split8(const uint4& xh, const uint4& xl, const uint4& yh, const uint4& yl,
+                                           uint4& hi, uint4& lo) {
+  const uint32_t a[4] = {xh.x, xh.y, xh.z, xh.w}, b[4] = {xl.x, xl.y, xl.z, xl.w};
+  const uint32_t c[4] = {yh.x, yh.y, yh.z, yh.w}, d[4] = {yl.x, yl.y, yl.z, yl.w};
+  uint32_t h[4], l[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const __half2 p = *reinterpret_cast<const __half2*>(&a[i]), q = *reinterpret_cast<const __half2*>(&b[i]);
+    const __half2 r = *reinterpret_cast<const __half2*>(&c[i]), s = *reinterpret_cast<const __half2*>(&d[i]);
+    const __half2 u = __hmul2(p, r);
+    const __half2 v = __hfma2(q, r, __hfma2(p, s, __hfma2(p, r, __hneg2(u))));
+    h[i] = *reinterpret_cast<const uint32_t*>(&u);
+    l[i] = *reinterpret_cast<const uint32_t*>(&v);
+  }
+  hi = make_uint4(h[0], h[1], h[2], h[3]);
+  lo = make_uint4(l[0], l[1], l[2], l[3]);
+}
+
+// A round of a 3D chunk: up to kRound samples, in z order, cut into groups of one
+// z block (first cell + 8) >> 3.  Every group starts at a table column that is
+// a multiple of 8; the round ends before column PAD.
+struct RoundGroups {
+  unsigned start[4];  // bit i: sample i starts a group
+  int pads[4];
+  int nround, ngrp;   // samples, groups
+  short col[kRound];  // table column of a sample
+  short gi[kRound + 1], gp[kRound], gz[kRound];  // groups: first sample, column, z block
+};
+
+__device__ __forceinline__ int z_block(float u, const Geom& g) { return ((int)ceilf(u - g.halfw) + 8) >> 3; }
+
+// u: the last-axis coordinates of the `left` samples that remain.  Whole CTA
+// (at least kRound threads); three barriers, the first before `rg` is read and
+// the last after it is complete.
+template <int PAD>
+__device__ __forceinline__ void round_groups(const float* __restrict__ u, int left, const Geom& g,
+                                             RoundGroups& rg) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const bool have = tid < kRound && tid < left;
+  int zb = 0;
+  bool start = false;
+  if (tid < kRound) {
+    if (have) {
+      zb = z_block(u[tid], g);
+      start = tid == 0 || zb != z_block(u[tid - 1], g);
+    }
+    const unsigned b = __ballot_sync(0xffffffffu, start);
+    if (lane == 0) rg.start[warp] = b;
+  }
+  __syncthreads();
+  // the group start at or before sample i of word w
+  auto start_of = [&](int w, unsigned below) {
+    while (!below) below = rg.start[--w];
+    return 32 * w + 31 - __clz(below);
+  };
+  int pad = 0, ord = 0;
+  if (tid < kRound) {
+    // empty columns before a group: the size of the last one up to a multiple of 8
+    if (start && tid > 0) pad = (start_of(warp, rg.start[warp] & ((1u << lane) - 1u)) - tid) & 7;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int q = __shfl_up_sync(0xffffffffu, pad, d);
+      if (lane >= d) pad += q;
+    }
+    if (lane == 31) rg.pads[warp] = pad;
+  }
+  __syncthreads();
+  if (tid < kRound) {
+    for (int w = 0; w < warp; ++w) {
+      pad += rg.pads[w];
+      ord += __popc(rg.start[w]);
+    }
+    const unsigned upto = rg.start[warp] & ((2u << lane) - 1u);
+    ord += __popc(upto) - 1;  // the sample's group
+    const int c = tid + pad;
+    const bool in = have && c < PAD;
+    rg.col[tid] = (short)(in ? c : -1);
+    if (in && start) {
+      rg.gi[ord] = (short)tid;
+      rg.gp[ord] = (short)c;
+      rg.gz[ord] = (short)zb;
+    }
+    bool last = in && (tid == kRound - 1 || tid + 1 == left);
+    if (in && !last) {  // the last sample before the columns run out
+      const bool next = rg.start[(tid + 1) >> 5] >> ((tid + 1) & 31) & 1;
+      last = c + 1 + (next ? (start_of(warp, upto) - (tid + 1)) & 7 : 0) >= PAD;
+    }
+    if (last) {
+      rg.nround = tid + 1;
+      rg.ngrp = ord + 1;
+      rg.gi[ord + 1] = (short)(tid + 1);
+    }
+  }
+  __syncthreads();
+}
 
 }  // namespace tc
 }  // namespace gbn

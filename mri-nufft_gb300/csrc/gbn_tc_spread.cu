@@ -13,16 +13,13 @@
 //       B = wz times the strength, the 16 slots a ring along z.
 //
 // Precision: every operand is split into two fp16 parts (x = hi + lo, 22 to
-// 23 bits) and D = Ah Bh + (Ah Bl + Al Bh).  The product of two split factors
-// is split in fp16 arithmetic: h = xh yh rounded, l = (xh yh - h) + xh yl +
-// xl yh, whose first term is exact.  The tensor core truncates when it adds to
-// an accumulator (measured: -5.6e-8 of the value for each MMA), so the two
-// cross terms, 2^-11 of the first, have accumulators of their own and the
-// Ah Bh chain is cut after a few steps of 16 samples (-2e-7 after 4 where every
-// term has one sign); longer sums continue in fp32, in registers (2D) or on
-// the fine grid (3D).  A is scaled to
-// 2^15 and B to 2^13 .. 2^15 over the largest strength, which keeps the fp16
-// parts' absolute floor at 2^-32 of the largest value.
+// 23 bits) and D = Ah Bh + (Ah Bl + Al Bh).  The tensor core truncates when it
+// adds to an accumulator (measured: -5.4e-8 of the value for each step of 16
+// samples), so the two cross terms, 2^-11 of the first, have accumulators of
+// their own, the Ah Bh chain is at most 8 steps long (longer sums continue in
+// fp32 on the fine grid), and the mean loss of its steps is given back.  A is
+// scaled to 2^15 and B to 2^13 .. 2^15 over the largest strength, which keeps
+// the fp16 parts' absolute floor at 2^-32 of the largest value.
 #include "gbn_internal.cuh"
 #include "gbn_tc.cuh"
 
@@ -33,54 +30,6 @@ namespace {
 using namespace tc;
 
 constexpr int kThreads = 256;
-// mean relative loss of an accumulator for each step that truncates it, given
-// back with the cross terms
-constexpr float kTrunc = 6e-8f;
-// scales: x, y (or z) weights 2^8, 2^7; strengths 2^(6 - e)
-constexpr float kScaleX = 256.0f, kScaleY = 128.0f, kScaleC = 64.0f;
-
-// the w <= 7 kernel weights t0 .. t0 + N - 1 of coordinate u; returns the first cell
-template <int N>
-__device__ __forceinline__ int weights_part(float u, const Geom& g, int t0, float (&wt)[N]) {
-  const int i0 = (int)ceilf(u - g.halfw);
-  const float x0 = (float)i0 - u;
-#pragma unroll
-  for (int t = 0; t < N; ++t)
-    wt[t] = t0 + t < g.w ? es_eval(x0 + (float)(t0 + t), g.beta, g.inv_halfw) : 0.f;
-  return i0;
-}
-
-__device__ __forceinline__ int wrap_once(int i, int n) {
-  const int m = i < 0 ? i + n : (i >= n ? i - n : i);
-  return (unsigned)m < (unsigned)n ? m : wrap_idx(i, n);
-}
-
-// v = hi + lo, stored as halves `lo_off` bytes apart
-__device__ __forceinline__ void put_split(unsigned char* p, int lo_off, float v) {
-  const __half h = __float2half_rn(v);
-  *reinterpret_cast<__half*>(p) = h;
-  *reinterpret_cast<__half*>(p + lo_off) = __float2half_rn(v - __half2float(h));
-}
-
-// the split product of two split factors, 8 samples
-__device__ __forceinline__ void mul_split8(const uint4& xh, const uint4& xl, const uint4& yh, const uint4& yl,
-                                           uint4& hi, uint4& lo) {
-  const uint32_t a[4] = {xh.x, xh.y, xh.z, xh.w}, b[4] = {xl.x, xl.y, xl.z, xl.w};
-  const uint32_t c[4] = {yh.x, yh.y, yh.z, yh.w}, d[4] = {yl.x, yl.y, yl.z, yl.w};
-  uint32_t h[4], l[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const __half2 p = *reinterpret_cast<const __half2*>(&a[i]), q = *reinterpret_cast<const __half2*>(&b[i]);
-    const __half2 r = *reinterpret_cast<const __half2*>(&c[i]), s = *reinterpret_cast<const __half2*>(&d[i]);
-    const __half2 u = __hmul2(p, r);
-    const __half2 v = __hfma2(q, r, __hfma2(p, s, __hfma2(p, r, __hneg2(u))));
-    h[i] = *reinterpret_cast<const uint32_t*>(&u);
-    l[i] = *reinterpret_cast<const uint32_t*>(&v);
-  }
-  hi = make_uint4(h[0], h[1], h[2], h[3]);
-  lo = make_uint4(l[0], l[1], l[2], l[3]);
-}
-
 // ---------------------------------------------------------------------------
 // 2D.  CTA = (chunk of <= 128 samples of one tile, group of TG transforms).
 // Cell (x, y) of the tile is row 8 x + (y >> 1) of M tile (y & 1), so that a
@@ -319,8 +268,7 @@ __global__ void __launch_bounds__(kThreads, 2) spread_tc2d_kernel(SpreadArgs a, 
 // ---------------------------------------------------------------------------
 constexpr int kChunk3 = kTcChunk3;
 constexpr int kCoils3 = 4;
-constexpr int kRows = 11;                      // cross-section rows per axis
-constexpr int kRound = 128;                    // samples of a round
+constexpr int kRows = kTcRows;
 constexpr int kPad = 192;                      // table columns of a round
 constexpr int kTabLo = 2 * kPad;               // hi -> lo part of a table row (bytes)
 constexpr int kTabP = 4 * kPad + 16;           // row pitch; an odd number of 16-byte units
@@ -338,11 +286,7 @@ __global__ void __launch_bounds__(kThreads, 2) spread_tc3d_kernel(SpreadArgs a, 
   __shared__ uint32_t s_tmem;
   __shared__ int s_row[128];
   __shared__ unsigned s_max[kCoils3];
-  __shared__ unsigned s_start[4];                // bit i: sample i of the round starts a group
-  __shared__ int s_pads[4];
-  __shared__ int s_nround, s_ngrp;
-  __shared__ short s_col[kRound];                // table column of a sample
-  __shared__ short s_gi[kRound + 1], s_gp[kRound], s_gz[kRound];  // groups: sample, column, z block
+  __shared__ RoundGroups rg;
 
   const Geom& g = a.g;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -451,80 +395,17 @@ __global__ void __launch_bounds__(kThreads, 2) spread_tc3d_kernel(SpreadArgs a, 
   bool ok = true;
 
   for (int s0 = 0; s0 < cnt;) {
-    // -- groups of the round: threads 0..127, sample s0 + tid
-    int zb = 0;
-    bool start = false;
-    const bool have = tid < kRound && s0 + tid < cnt;
-    if (tid < kRound) {
-      if (have) {
-        zb = ((int)ceilf(a.s.u[2][p0 + s0 + tid] - g.halfw) + 8) >> 3;
-        start = tid == 0 || zb != ((int)ceilf(a.s.u[2][p0 + s0 + tid - 1] - g.halfw) + 8) >> 3;
-      }
-      const unsigned b = __ballot_sync(0xffffffffu, start);
-      if (lane == 0) s_start[warp] = b;
-    }
     // the tables of the last round are consumed (its last block's barrier)
     for (int i = tid; i < kTabRows * kTabP / 16; i += kThreads)
       reinterpret_cast<uint4*>(s_tab)[i] = make_uint4(0, 0, 0, 0);
-    __syncthreads();
-    int pad = 0, ord = 0;
-    if (tid < kRound) {
-      if (start && tid > 0) {  // empty columns before this group: the last one's size to a multiple of 8
-        int w = warp;
-        unsigned below = s_start[w] & ((1u << lane) - 1u);
-        while (!below) below = s_start[--w];
-        pad = (32 * w + 31 - __clz(below) - tid) & 7;
-      }
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const int q = __shfl_up_sync(0xffffffffu, pad, d);
-        if (lane >= d) pad += q;
-      }
-      if (lane == 31) s_pads[warp] = pad;
-    }
-    __syncthreads();
-    if (tid < kRound) {
-      for (int w = 0; w < warp; ++w) {
-        pad += s_pads[w];
-        ord += __popc(s_start[w]);
-      }
-      ord += __popc(s_start[warp] & ((2u << lane) - 1u)) - 1;  // the sample's group
-      const int c = tid + pad;
-      const bool in = have && c < kPad;
-      s_col[tid] = (short)(in ? c : -1);
-      if (in && start) {
-        s_gi[ord] = (short)tid;
-        s_gp[ord] = (short)c;
-        s_gz[ord] = (short)zb;
-      }
-      // the last sample that fits ends the round
-      const int cn = tid + 1 + pad;  // at least the next sample's column
-      bool last = in && (tid == kRound - 1 || s0 + tid + 1 == cnt);
-      if (in && !last) {
-        const int w = (tid + 1) >> 5, ln = (tid + 1) & 31;
-        int p = 0;
-        if (s_start[w] >> ln & 1) {  // the next sample starts a group
-          unsigned below = s_start[warp] & ((2u << lane) - 1u);
-          int wb = warp;
-          while (!below) below = s_start[--wb];
-          p = (32 * wb + 31 - __clz(below) - (tid + 1)) & 7;
-        }
-        last = cn + p >= kPad;
-      }
-      if (last) {
-        s_nround = tid + 1;
-        s_ngrp = ord + 1;
-        s_gi[ord + 1] = (short)(tid + 1);
-      }
-    }
-    __syncthreads();
-    const int nr = s_nround, ng = s_ngrp;
+    round_groups<kPad>(a.s.u[2] + p0 + s0, cnt - s0, g, rg);
+    const int nr = rg.nround, ng = rg.ngrp;
     // -- tables: weights of an axis, then strengths of a coil, 32 samples a warp
     for (int q = warp; q < 12 + 4 * kCoils3; q += kThreads / 32) {
       const int i = 32 * (q & 3) + lane;
       if (i >= nr) continue;
       const int pos = p0 + s0 + i;
-      unsigned char* const t0 = s_tab + 2 * s_col[i];
+      unsigned char* const t0 = s_tab + 2 * rg.col[i];
       if (q < 12) {
         const int d = q >> 2;
         float wt[7];
@@ -556,7 +437,7 @@ __global__ void __launch_bounds__(kThreads, 2) spread_tc3d_kernel(SpreadArgs a, 
     __syncthreads();
 
     for (int gr = 0; gr < ng; ++gr) {
-      const int ngr = s_gi[gr + 1] - s_gi[gr], blk = s_gz[gr], pc = s_gp[gr];
+      const int ngr = rg.gi[gr + 1] - rg.gi[gr], blk = rg.gz[gr], pc = rg.gp[gr];
       for (int b = 0; b < ngr; b += 32, ++it) {
         const int no = (imin(32, ngr - b) + 7) >> 3;  // octets with samples
         const int nk = (no + 1) >> 1;

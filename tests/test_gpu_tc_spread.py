@@ -51,3 +51,30 @@ def test_against_fp32_atomics(gpu_pkg, monkeypatch, shape, M, C, eps):
         out.append(np.asarray(op.adj_op(y)))
     for c in range(C):
         assert rel_l2(out[0][0, c], out[1][0, c]) < BOUND, c
+
+
+@pytest.mark.parametrize("eps", [1e-1, 1e-2, 1e-3, 1e-4, 1e-5, 1e-6])
+@pytest.mark.parametrize("shape,M,C", [((30, 47), 2600, 2), ((251, 16), 3001, 17), ((64, 96), 517, 35),
+                                       ((250, 256), 900, 66), ((256, 251), 20000, 27),
+                                       ((256, 256), 3000, 25), ((20, 18, 16), 5000, 3)])
+def test_interp_against_fp32_gather(gpu_pkg, monkeypatch, shape, M, C, eps):
+    """The tensor-core interpolation (op, data consistency with density) against
+    the per-sample FP32 one, by the same bound; images of scales 1e-6 .. 1e6,
+    transform counts that leave partial groups (32, 64 per CTA); sizes and counts
+    that keep the FP32 kernels too (other grids than 512^2, up to 24 transforms)."""
+    rng = np.random.default_rng(M + C + 1)
+    k = _samples(len(shape), M, rng)
+    x = rng.standard_normal((1, C, *shape)) + 1j * rng.standard_normal((1, C, *shape))
+    x *= 10.0 ** np.linspace(-6, 6, C).reshape(-1, *[1] * len(shape))
+    x = x.astype(np.complex64)
+    dens = rng.uniform(0.5, 1.5, M).astype(np.float32)
+    out = []
+    for interp in ("auto", "gm"):
+        monkeypatch.setenv("GBN_SPREAD", "mma")
+        monkeypatch.setenv("GBN_INTERP", interp)
+        op = gpu_pkg.MRIGB300(k, shape, n_coils=C, density=dens, squeeze_dims=False, eps=eps)
+        y = np.asarray(op.op(x))
+        out.append((y, np.asarray(op.data_consistency(x, 0.25 * y))))
+    for c in range(C):
+        assert rel_l2(out[0][0][0, c], out[1][0][0, c]) < BOUND, c
+        assert rel_l2(out[0][1][0, c], out[1][1][0, c]) < 2 * BOUND, c
