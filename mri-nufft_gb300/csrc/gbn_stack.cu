@@ -13,6 +13,13 @@
 //            inverse cuFFT along z,
 //            crop  img[x][y][z] = sum_c conj(s_c) P[c][x][y][(z - h) mod Nz]
 //            (calibless: one image per coil).
+//
+// Stacks of up to about 128 planes do each direction in one kernel instead: 32
+// (x, y) columns of a CTA go through shared memory, the z transform is a sum over
+// Nz / R terms per plane after one radix-R step (R = 4, 2 or 1, the largest that
+// divides Nz), and the work stack is never written: 1.1 GB a direction instead of
+// 3.2 GB for 256 x 256 x 64 and 16 coils, op + adj around the 2D transforms 3.2 ->
+// 1.0 ms (floor at the copy bandwidth 0.33; the forward sum is FP32-bound).
 #include <cufft.h>
 
 #include <cmath>
@@ -124,6 +131,235 @@ __global__ void stack_crop_kernel(StackGeom g, const float2* __restrict__ P,
   }
 }
 
+// ---------------------------------------------------------------------------
+// One-kernel z transforms.  With n4 = Nz / R and z = z' + p n4 (positions of the
+// shifted axis), plane f = zpos is
+//   X[f] = sum_{z' < n4} W^(f z') t_{f mod R}[z'],  t_r[z'] = sum_p v[z' + p n4] i_R^(-r p),
+// i_R = exp(2 pi i / R).  `order` lists the kept planes by f mod R in groups of 8
+// of one residue (-1: padding), W[z'][j] = exp(-2 pi i f_j z' / Nz) (0: padding).
+// Lane = column throughout.
+// ---------------------------------------------------------------------------
+struct StackDft {
+  const float2* W;     // n4 x npad
+  const int* order;    // npad
+  int n4, npad;
+};
+constexpr int kDftCols = 32;
+constexpr int kDftThreads = 256;
+constexpr int kDftWarps = kDftThreads / 32;
+
+__device__ __forceinline__ float2 rot_m(float2 v, int q) {  // v * (-i)^q
+  switch (q & 3) {
+    case 0: return v;
+    case 1: return make_float2(v.y, -v.x);
+    case 2: return make_float2(-v.x, -v.y);
+    default: return make_float2(-v.y, v.x);
+  }
+}
+
+// grid: columns / 32, coils
+template <int R>
+__global__ void __launch_bounds__(kDftThreads)
+stack_fwd_dft_kernel(StackGeom g, StackDft d, const float2* __restrict__ img,
+                     const float2* __restrict__ smaps, float2* __restrict__ out, float scale) {
+  extern __shared__ __align__(16) float2 s_dft[];
+  float2* const s_w = s_dft;                       // [n4][npad]
+  float2* const s_v = s_w + d.n4 * d.npad;         // [nz][33]
+  constexpr int P = kDftCols + 1;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t col0 = (int64_t)blockIdx.x * kDftCols;
+  const int ncol = g.nxy - col0 < kDftCols ? (int)(g.nxy - col0) : kDftCols;
+  const int c = blockIdx.y;
+  for (int i = threadIdx.x; i < d.n4 * d.npad; i += kDftThreads) s_w[i] = d.W[i];
+  const float2* const src = (smaps ? img : img + (int64_t)c * g.nimg) + col0 * g.nz;
+  const float2* const map = smaps ? smaps + (int64_t)c * g.nimg + col0 * g.nz : nullptr;
+  for (int i = threadIdx.x; i < kDftCols * g.nz; i += kDftThreads) {
+    const int cl = i / g.nz, z = i - cl * g.nz;
+    float2 v = make_float2(0.f, 0.f);
+    if (cl < ncol) {
+      v = src[i];
+      if (map) v = cmul_(v, map[i]);
+    }
+    int zz = z - g.nz / 2;
+    if (zz < 0) zz += g.nz;
+    s_v[zz * P + cl] = v;
+  }
+  __syncthreads();
+  if (R > 1) {
+    for (int z = warp; z < d.n4; z += kDftWarps) {
+      float2 v[R], t[R];
+#pragma unroll
+      for (int p = 0; p < R; ++p) v[p] = s_v[(z + p * d.n4) * P + lane];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        t[r] = v[0];
+#pragma unroll
+        for (int p = 1; p < R; ++p) {
+          const float2 w = rot_m(v[p], (4 / R) * r * p);
+          t[r].x += w.x;
+          t[r].y += w.y;
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r) s_v[(z + r * d.n4) * P + lane] = t[r];
+    }
+    __syncthreads();
+  }
+  for (int j0 = 8 * warp; j0 < d.npad; j0 += 8 * kDftWarps) {
+    const int r = R == 1 ? 0 : d.order[j0] & (R - 1);  // the group's residue (low bits of order)
+    float2 acc[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[j] = make_float2(0.f, 0.f);
+    const float2* const t = s_v + r * d.n4 * P + lane;
+    for (int z = 0; z < d.n4; ++z) {
+      const float2 v = t[z * P];
+      const float2 iv = make_float2(-v.y, v.x);
+      const float4* const w4 = reinterpret_cast<const float4*>(s_w + z * d.npad + j0);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float4 w = w4[q];
+        acc[2 * q] = __ffma2_rn(make_float2(w.x, w.x), v, acc[2 * q]);
+        acc[2 * q] = __ffma2_rn(make_float2(w.y, w.y), iv, acc[2 * q]);
+        acc[2 * q + 1] = __ffma2_rn(make_float2(w.z, w.z), v, acc[2 * q + 1]);
+        acc[2 * q + 1] = __ffma2_rn(make_float2(w.w, w.w), iv, acc[2 * q + 1]);
+      }
+    }
+    if (lane < ncol) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int k = d.order[j0 + j] >> 2;
+        if (k >= 0)
+          out[((int64_t)c * g.nzi + k) * g.nxy + col0 + lane] = make_float2(acc[j].x * scale, acc[j].y * scale);
+      }
+    }
+  }
+}
+
+// grid: columns / 32 (SENSE: every coil in turn, summed), x coils without maps
+template <int R>
+__global__ void __launch_bounds__(kDftThreads)
+stack_adj_dft_kernel(StackGeom g, StackDft d, const float2* __restrict__ in,
+                     const float2* __restrict__ smaps, float2* __restrict__ img, int C, int accumulate,
+                     float scale) {
+  constexpr int ZP = 16 / R;  // z' of a warp: n4 <= 8 ZP
+  extern __shared__ __align__(16) float2 s_dft[];
+  float2* const s_w = s_dft;                            // [n4][npad]
+  float2* const s_in = s_w + d.n4 * d.npad;             // [npad][32]
+  float2* const s_m = s_in + d.npad * kDftCols;         // [32][nz + 1], maps, then the result
+  const int mp = g.nz + 1 + (g.nz & 1);                 // odd pitch
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t col0 = (int64_t)blockIdx.x * kDftCols;
+  const int ncol = g.nxy - col0 < kDftCols ? (int)(g.nxy - col0) : kDftCols;
+  const int cb = smaps ? 0 : blockIdx.y, ce = smaps ? C : cb + 1;
+  for (int i = threadIdx.x; i < d.n4 * d.npad; i += kDftThreads) s_w[i] = d.W[i];
+  float2 acc[ZP][R];
+#pragma unroll
+  for (int q = 0; q < ZP; ++q)
+#pragma unroll
+    for (int p = 0; p < R; ++p) acc[q][p] = make_float2(0.f, 0.f);
+  for (int c = cb; c < ce; ++c) {
+    __syncthreads();  // the last coil's planes and maps are consumed
+    for (int j = warp; j < d.npad; j += kDftWarps) {
+      const int k = d.order[j] >> 2;
+      float2 v = make_float2(0.f, 0.f);
+      if (k >= 0 && lane < ncol) v = in[((int64_t)c * g.nzi + k) * g.nxy + col0 + lane];
+      s_in[j * kDftCols + lane] = v;
+    }
+    if (smaps) {
+      const float2* const map = smaps + (int64_t)c * g.nimg + col0 * g.nz;
+      for (int i = threadIdx.x; i < ncol * g.nz; i += kDftThreads) {
+        const int cl = i / g.nz;
+        s_m[cl * mp + (i - cl * g.nz)] = map[i];
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < ZP; ++q) {
+      const int z = warp + kDftWarps * q;
+      if (z >= d.n4) break;
+      float2 S[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) S[r] = make_float2(0.f, 0.f);
+      for (int j0 = 0; j0 < d.npad; j0 += 8) {
+        float2 t = make_float2(0.f, 0.f);
+        const float4* const w4 = reinterpret_cast<const float4*>(s_w + z * d.npad + j0);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {  // conj(W) v
+          const float4 w = w4[e];
+          const float2 a = s_in[(j0 + 2 * e) * kDftCols + lane], b = s_in[(j0 + 2 * e + 1) * kDftCols + lane];
+          t = __ffma2_rn(make_float2(w.x, w.x), a, t);
+          t = __ffma2_rn(make_float2(w.y, w.y), make_float2(a.y, -a.x), t);
+          t = __ffma2_rn(make_float2(w.z, w.z), b, t);
+          t = __ffma2_rn(make_float2(w.w, w.w), make_float2(b.y, -b.x), t);
+        }
+        const int r = R == 1 ? 0 : d.order[j0] & (R - 1);
+#pragma unroll
+        for (int e = 0; e < R; ++e)
+          if (r == e) {
+            S[e].x += t.x;
+            S[e].y += t.y;
+          }
+      }
+#pragma unroll
+      for (int p = 0; p < R; ++p) {
+        float2 v = S[0];
+#pragma unroll
+        for (int r = 1; r < R; ++r) {
+          const float2 w = rot_m(S[r], 4 - (4 / R) * r * p % 4);  // S_r i_R^(r p)
+          v.x += w.x;
+          v.y += w.y;
+        }
+        if (smaps) {
+          int zi = z + p * d.n4 + g.nz / 2;
+          if (zi >= g.nz) zi -= g.nz;
+          if (lane < ncol) v = cmulc_(s_m[lane * mp + zi], v);
+        }
+        acc[q][p].x += v.x;
+        acc[q][p].y += v.y;
+      }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < ZP; ++q) {
+    const int z = warp + kDftWarps * q;
+    if (z >= d.n4) break;
+#pragma unroll
+    for (int p = 0; p < R; ++p) {
+      int zi = z + p * d.n4 + g.nz / 2;
+      if (zi >= g.nz) zi -= g.nz;
+      s_m[lane * mp + zi] = make_float2(acc[q][p].x * scale, acc[q][p].y * scale);
+    }
+  }
+  __syncthreads();
+  float2* const dst = img + (int64_t)cb * g.nimg + col0 * g.nz;
+  for (int i = threadIdx.x; i < ncol * g.nz; i += kDftThreads) {
+    const int cl = i / g.nz;
+    float2 v = s_m[cl * mp + (i - cl * g.nz)];
+    if (accumulate) {
+      v.x += dst[i].x;
+      v.y += dst[i].y;
+    }
+    dst[i] = v;
+  }
+}
+
+template <int R>
+cudaError_t dft_fwd(const StackGeom& g, const StackDft& d, const float2* img, const float2* smaps, float2* out,
+                    int C, float scale, size_t smem, cudaStream_t st) {
+  stack_fwd_dft_kernel<R><<<dim3((unsigned)((g.nxy + kDftCols - 1) / kDftCols), C), kDftThreads, smem, st>>>(
+      g, d, img, smaps, out, scale);
+  return cudaGetLastError();
+}
+template <int R>
+cudaError_t dft_adj(const StackGeom& g, const StackDft& d, const float2* in, const float2* smaps, float2* img,
+                    int C, int accumulate, float scale, size_t smem, cudaStream_t st) {
+  stack_adj_dft_kernel<R>
+      <<<dim3((unsigned)((g.nxy + kDftCols - 1) / kDftCols), smaps ? 1 : C), kDftThreads, smem, st>>>(
+          g, d, in, smaps, img, C, accumulate, scale);
+  return cudaGetLastError();
+}
+
 unsigned blocks_for(int64_t n) {
   int64_t b = (n + 255) / 256;
   if (b < 1) b = 1;
@@ -143,6 +379,11 @@ struct gbn_stack_s {
   float2* P = nullptr;     // C x nx x ny x nz work stack
   int64_t pcap = 0;        // cells of P
   std::map<int, cufftHandle> ffts;
+  int radix = 0;           // one-kernel z transforms: R (0: pad, cuFFT and gather)
+  StackDft dft{};
+  float2* W = nullptr;
+  int* order = nullptr;
+  size_t smem_fwd = 0, smem_adj = 0;
   ~gbn_stack_s() {
     int prev = -1;
     cudaGetDevice(&prev);
@@ -150,6 +391,8 @@ struct gbn_stack_s {
     for (auto& kv : ffts) cufftDestroy(kv.second);
     if (zpos) cudaFree(zpos);
     if (P) cudaFree(P);
+    if (W) cudaFree(W);
+    if (order) cudaFree(order);
     if (prev >= 0 && prev != device) cudaSetDevice(prev);
   }
 };
@@ -217,6 +460,62 @@ int exec_z(cufftHandle h, float2* P, int dir, cudaStream_t st) {
   return GBN_OK;
 }
 
+// Tables of the one-kernel z transforms when the stack fits them: distinct planes
+// (a repeated one is written by an unspecified copy in the scatter) and tables
+// and columns within 96 KB of shared memory.
+int stack_setup_dft(gbn_stack s, const std::vector<int>& pos) {
+  const StackGeom& g = s->g;
+  const int R = g.nz % 4 == 0 ? 4 : g.nz % 2 == 0 ? 2 : 1;
+  const int n4 = g.nz / R;
+  if (n4 > 8 * (16 / R)) return GBN_OK;
+  std::vector<char> seen(g.nz, 0);
+  std::vector<int> order, freq;
+  for (int f : pos) {
+    if (seen[f]) return GBN_OK;
+    seen[f] = 1;
+  }
+  for (int r = 0; r < R; ++r) {
+    for (size_t k = 0; k < pos.size(); ++k)
+      if (pos[k] % R == r) {
+        order.push_back((int)k * 4 + r);
+        freq.push_back(pos[k]);
+      }
+    while (order.size() % 8) {
+      order.push_back(-4 + r);  // >> 2 is -1, the residue stays in the low bits
+      freq.push_back(-1);
+    }
+  }
+  const int npad = (int)order.size();
+  const size_t wb = (size_t)n4 * npad * sizeof(float2);
+  s->smem_fwd = wb + (size_t)g.nz * (kDftCols + 1) * sizeof(float2);
+  s->smem_adj = wb + (size_t)npad * kDftCols * sizeof(float2) + (size_t)kDftCols * (g.nz + 2) * sizeof(float2);
+  if (s->smem_fwd > 96 * 1024 || s->smem_adj > 96 * 1024) return GBN_OK;
+  std::vector<float2> W((size_t)n4 * npad, make_float2(0.f, 0.f));
+  const double pi = 3.14159265358979323846;
+  for (int z = 0; z < n4; ++z)
+    for (int j = 0; j < npad; ++j)
+      if (freq[j] >= 0) {
+        const double a = 2.0 * pi * (double)((int64_t)freq[j] * z % g.nz) / g.nz;
+        W[(size_t)z * npad + j] = make_float2((float)std::cos(a), (float)-std::sin(a));
+      }
+  int rc = ck_cuda(cudaMalloc(&s->W, wb), "stack z table");
+  if (!rc) rc = ck_cuda(cudaMemcpy(s->W, W.data(), wb, cudaMemcpyHostToDevice), "stack z table");
+  if (!rc) rc = ck_cuda(cudaMalloc(&s->order, sizeof(int) * npad), "stack plane order");
+  if (!rc)
+    rc = ck_cuda(cudaMemcpy(s->order, order.data(), sizeof(int) * npad, cudaMemcpyHostToDevice),
+                 "stack plane order");
+  for (const void* k : {(const void*)stack_fwd_dft_kernel<1>, (const void*)stack_fwd_dft_kernel<2>,
+                        (const void*)stack_fwd_dft_kernel<4>, (const void*)stack_adj_dft_kernel<1>,
+                        (const void*)stack_adj_dft_kernel<2>, (const void*)stack_adj_dft_kernel<4>})
+    if (!rc)
+      rc = ck_cuda(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024),
+                   "stack kernel attributes");
+  if (rc) return rc;
+  s->dft = StackDft{s->W, s->order, n4, npad};
+  s->radix = R;
+  return GBN_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -248,6 +547,7 @@ int gbn_stack_create(const int64_t* shape, const int* z_index, int n_index, int 
   if (!rc)
     rc = ck_cuda(cudaMemcpy(s->zpos, pos.data(), sizeof(int) * n_index, cudaMemcpyHostToDevice),
                  "stack z positions");
+  if (!rc) rc = stack_setup_dft(s, pos);
   if (rc) {
     delete s;
     return rc;
@@ -261,15 +561,23 @@ int gbn_stack_fwd(gbn_stack s, const void* img, const void* smaps, void* out, in
   if (!s || !img || !out || C < 1) return stack_fail(GBN_ERR_ARG, "invalid stack arguments");
   DevSwitch dg(s->device);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  const StackGeom& g = s->g;
+  const float scale = (float)(1.0 / std::sqrt(2.0 * g.nz));
+  if (s->radix && C <= 65535) {
+    const float2 *x = static_cast<const float2*>(img), *m = static_cast<const float2*>(smaps);
+    float2* const y = static_cast<float2*>(out);
+    return ck_cuda(s->radix == 4   ? dft_fwd<4>(g, s->dft, x, m, y, C, scale, s->smem_fwd, st)
+                   : s->radix == 2 ? dft_fwd<2>(g, s->dft, x, m, y, C, scale, s->smem_fwd, st)
+                                   : dft_fwd<1>(g, s->dft, x, m, y, C, scale, s->smem_fwd, st),
+                   "stack forward");
+  }
   cufftHandle h;
   int rc = stack_prepare(s, C, &h);
   if (rc) return rc;
-  const StackGeom& g = s->g;
   stack_pad_kernel<<<blocks_for((int64_t)C * g.nimg), 256, 0, st>>>(
       g, static_cast<const float2*>(img), static_cast<const float2*>(smaps), s->P, C);
   if ((rc = ck_cuda(cudaGetLastError(), "stack pad"))) return rc;
   if ((rc = exec_z(h, s->P, CUFFT_FORWARD, st))) return rc;
-  const float scale = (float)(1.0 / std::sqrt(2.0 * g.nz));
   stack_gather_kernel<<<blocks_for((int64_t)C * g.nzi * g.nxy), 256, 0, st>>>(
       g, s->P, s->zpos, static_cast<float2*>(out), C, scale);
   return ck_cuda(cudaGetLastError(), "stack gather");
@@ -280,13 +588,21 @@ int gbn_stack_adj(gbn_stack s, const void* in, const void* smaps, void* img, int
   if (!s || !in || !img || C < 1) return stack_fail(GBN_ERR_ARG, "invalid stack arguments");
   DevSwitch dg(s->device);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  const StackGeom& g = s->g;
+  const float scale = (float)(1.0 / std::sqrt(2.0 * g.nz));
+  if (s->radix && C <= 65535) {
+    const float2 *y = static_cast<const float2*>(in), *m = static_cast<const float2*>(smaps);
+    float2* const x = static_cast<float2*>(img);
+    return ck_cuda(s->radix == 4   ? dft_adj<4>(g, s->dft, y, m, x, C, accumulate, scale, s->smem_adj, st)
+                   : s->radix == 2 ? dft_adj<2>(g, s->dft, y, m, x, C, accumulate, scale, s->smem_adj, st)
+                                   : dft_adj<1>(g, s->dft, y, m, x, C, accumulate, scale, s->smem_adj, st),
+                   "stack adjoint");
+  }
   cufftHandle h;
   int rc = stack_prepare(s, C, &h);
   if (rc) return rc;
-  const StackGeom& g = s->g;
   if ((rc = ck_cuda(cudaMemsetAsync(s->P, 0, sizeof(float2) * (size_t)C * g.nimg, st), "stack zero")))
     return rc;
-  const float scale = (float)(1.0 / std::sqrt(2.0 * g.nz));
   stack_scatter_kernel<<<blocks_for((int64_t)C * g.nzi * g.nxy), 256, 0, st>>>(
       g, static_cast<const float2*>(in), s->zpos, s->P, C, scale);
   if ((rc = ck_cuda(cudaGetLastError(), "stack scatter"))) return rc;
