@@ -677,16 +677,15 @@ GBN_UNROLL
 }
 
 // ---------------------------------------------------------------------------
-// Warp-cooperative interpolation straight from the fine grid (w = 7).
+// Warp-cooperative interpolation straight from the fine grid (w <= 7).
 // Eight lanes serve one sample: lane l reads footprint cells along the last
 // axis at offset l (7 contiguous float2 per row, i.e. 56 coalesced bytes per
 // sample), so one warp instruction loads the rows of four samples in a few
 // sectors; partial sums are combined with three butterfly shuffles.  The
 // kernel weights of a sample stay in registers for every transform.
 // ---------------------------------------------------------------------------
-template <int DIM>
+template <int DIM, int W = 7>
 __device__ __forceinline__ void interp_wc_body(const InterpArgs& a, const int64_t warp_id) {
-  constexpr int W = 7;
   const Geom& g = a.g;
   const int lane = threadIdx.x & 31;
   const int sub = lane >> 3, l = lane & 7;
@@ -775,10 +774,10 @@ __device__ __forceinline__ void interp_wc_body(const InterpArgs& a, const int64_
   }
 }
 
-template <int DIM>
+template <int DIM, int W>
 __global__ void __launch_bounds__(GBN_THREADS, 4)
 interp_wc_kernel(InterpArgs a) {
-  interp_wc_body<DIM>(a, ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  interp_wc_body<DIM, W>(a, ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
 }
 
 // ---------------------------------------------------------------------------
@@ -1944,6 +1943,65 @@ GBN_UNROLL
   }
 }
 
+// ---------------------------------------------------------------------------
+// The same in 2D straight from the fine grid (w <= 7): eight lanes serve one
+// sample, lane l its footprint cells at offset l of the last axis.  Weights and
+// derivatives stay in registers for every transform, the products with the
+// cotangents are summed per lane over all transforms and the lanes reduced once.
+// Bound by L1 and issue like interp_wc; against the tile kernel, which evaluates
+// the weights again for every transform and waits at its tile barriers: 131 072
+// samples, 8 transforms 166 -> 56 us.
+// ---------------------------------------------------------------------------
+template <int W>
+__global__ void __launch_bounds__(GBN_THREADS, 4)
+grad_wc2d_kernel(GradArgs a, int conj_a) {
+  const Geom& g = a.g;
+  const int lane = threadIdx.x & 31;
+  const int l = lane & 7;
+  const int64_t pos = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 4 + (lane >> 3);
+  const bool valid = pos < a.s.M;
+  float gx = 0.f, gy = 0.f;
+  int j = 0;
+  if (valid && l < W) {
+    j = a.s.perm[pos];
+    float w0[W], d0[W];
+    const int i0 = weights_rt_d<W>(a.s.u[0][pos], g, w0, d0);
+    const float u1 = a.s.u[1][pos];
+    const int i1 = (int)ceilf(u1 - g.halfw);
+    const float x1 = (float)(i1 + l) - u1;
+    const float wl = es_eval(x1, g.beta, g.inv_halfw), dl = -es_deriv(x1, g.beta, g.inv_halfw);
+    int rb[W];
+#pragma unroll
+    for (int t = 0; t < W; ++t) rb[t] = wrap_idx(i0 + t, g.nf[0]) * g.nf[1];
+    const float2* base = a.fine + wrap_idx(i1 + l, g.nf[1]);
+    const float2* dy = a.dy + j;
+    for (int c = 0; c < a.ntr; ++c, base += g.G, dy += a.s.M) {
+      float2 s = make_float2(0.f, 0.f), d = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int t = 0; t < W; ++t) {
+        const float2 v = __ldg(base + rb[t]);
+        s = __ffma2_rn(make_float2(w0[t], w0[t]), v, s);
+        d = __ffma2_rn(make_float2(d0[t], d0[t]), v, d);
+      }
+      float2 av = *dy;
+      if (conj_a) av.y = -av.y;
+      gx += av.x * d.x - av.y * d.y;  // Re(av (d / du0))
+      gy += av.x * s.x - av.y * s.y;
+    }
+    gx *= wl;
+    gy *= dl;
+  }
+#pragma unroll
+  for (int o = 1; o < 8; o <<= 1) {
+    gx += __shfl_xor_sync(0xffffffffu, gx, o);
+    gy += __shfl_xor_sync(0xffffffffu, gy, o);
+  }
+  if (valid && l == 0) {
+    a.grad[(int64_t)j * 2] += a.scale * g.uscale[0] * gx;
+    a.grad[(int64_t)j * 2 + 1] += a.scale * g.uscale[1] * gy;
+  }
+}
+
 template <int DIM, int W, int CG>
 cudaError_t launch_interp_t(const InterpArgs& a, cudaStream_t st) {
   if (a.s.nsub == 0) return cudaSuccess;
@@ -2044,9 +2102,16 @@ cudaError_t launch_grad_t(const GradArgs& a, int conj_a, cudaStream_t st) {
 
 template <int DIM, int CG>
 cudaError_t dispatch_interp_w(const InterpArgs& a, cudaStream_t st) {
-  // w = 7 is the width of mri-nufft's default eps = 1e-6 at upsampfac 2;
-  // every other width runs the runtime-width kernel.
+  // w = 7 is the width of mri-nufft's default eps = 1e-6 at upsampfac 2; 4 to 6
+  // those of 1e-3 .. 1e-5 (3D, 8 coils, 786 432 samples, w = 5: 1.08 ms with the
+  // runtime-width kernel, whose 16-entry weight arrays and tests cost more than
+  // the 125 cells; 0.50 unrolled).  Every other width runs the runtime-width kernel.
   if (a.g.w == 7) return launch_interp_t<DIM, 7, CG>(a, st);
+  if constexpr (DIM == 3 && CG == 1) {
+    if (a.g.w == 6) return launch_interp_t<DIM, 6, CG>(a, st);
+    if (a.g.w == 5) return launch_interp_t<DIM, 5, CG>(a, st);
+    if (a.g.w == 4) return launch_interp_t<DIM, 4, CG>(a, st);
+  }
   return launch_interp_t<DIM, 0, CG>(a, st);
 }
 
@@ -2072,12 +2137,12 @@ cudaError_t launch_interp_db_t(const InterpArgs& a, cudaStream_t st) {
   return cudaGetLastError();
 }
 
-template <int DIM>
+template <int DIM, int W = 7>
 cudaError_t launch_interp_wc_t(const InterpArgs& a, cudaStream_t st) {
   if (a.s.M == 0) return cudaSuccess;
   const int64_t warps = (a.s.M + 3) / 4;
   const unsigned blocks = (unsigned)((warps * 32 + GBN_THREADS - 1) / GBN_THREADS);
-  interp_wc_kernel<DIM><<<blocks, GBN_THREADS, 0, st>>>(a);
+  interp_wc_kernel<DIM, W><<<blocks, GBN_THREADS, 0, st>>>(a);
   return cudaGetLastError();
 }
 
@@ -2098,6 +2163,13 @@ cudaError_t dispatch_interp(const InterpArgs& a, cudaStream_t st) {
   // stack-of-stars, 2.7x before it); 3D to tiles.  GBN_INTERP=tile forces tiles.
   if (a.g.w == 7 && (a.g.method_interp == 4 || (DIM == 2 && a.g.method_interp == 0)))
     return launch_interp_wc_t<DIM>(a, st);
+  if constexpr (DIM == 2) {  // the widths of eps 1e-3 .. 1e-5
+    if (a.g.method_interp == 0) {
+      if (a.g.w == 6) return launch_interp_wc_t<2, 6>(a, st);
+      if (a.g.w == 5) return launch_interp_wc_t<2, 5>(a, st);
+      if (a.g.w == 4) return launch_interp_wc_t<2, 4>(a, st);
+    }
+  }
   if (DIM == 3 && a.g.method_interp == 5 && a.g.w == 7 && a.s.maxsub <= kTwcMaxSub)
     return launch_interp_twc(a, st);
   // default for the w = 7 kernel: double-buffered tiles with register weights
@@ -2140,9 +2212,24 @@ cudaError_t dispatch_spread(const SpreadArgs& a, cudaStream_t st) {
   return launch_spread_gm_t<DIM, 0>(a, st);
 }
 
+template <int W>
+cudaError_t launch_grad_wc2d(const GradArgs& a, cudaStream_t st) {
+  if (a.s.M == 0) return cudaSuccess;
+  const int64_t warps = (a.s.M + 3) / 4;
+  const unsigned blocks = (unsigned)((warps * 32 + GBN_THREADS - 1) / GBN_THREADS);
+  grad_wc2d_kernel<W><<<blocks, GBN_THREADS, 0, st>>>(a, a.conj_a);
+  return cudaGetLastError();
+}
+
 template <int DIM>
 cudaError_t dispatch_grad(const GradArgs& a, cudaStream_t st) {
-  // runtime-width kernel: the derivative path is not the throughput path
+  if constexpr (DIM == 2) {
+    if (a.g.w == 7) return launch_grad_wc2d<7>(a, st);
+    if (a.g.w == 6) return launch_grad_wc2d<6>(a, st);
+    if (a.g.w == 5) return launch_grad_wc2d<5>(a, st);
+    if (a.g.w == 4) return launch_grad_wc2d<4>(a, st);
+  }
+  // 3D and other widths: runtime-width tiles
   return launch_grad_t<DIM, 0>(a, a.conj_a, st);
 }
 
