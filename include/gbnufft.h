@@ -89,6 +89,12 @@ int gbn_plan_device_bytes(gbn_plan plan, int64_t* bytes);
 int gbn_plan_tune(gbn_plan plan, const int* bins, int interp_method, int maxsub_cap);
 
 /*
+ * Raise the number of transforms of a pass to at least `ntrans` (larger fine
+ * grids; points and tuning are kept, the old grids are freed with the plan).
+ */
+int gbn_plan_reserve(gbn_plan plan, int ntrans);
+
+/*
  * Set the non-uniform points: M samples, one float32 device array per image
  * axis (k2 ignored in 2D).  Bin-sorts the points on the device.  Replaces
  * Plan.setpts (finufft.py:55-62, cufinufft.py:94-113).

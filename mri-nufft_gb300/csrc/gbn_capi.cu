@@ -160,6 +160,7 @@ struct gbn_plan_s {
   float* dec[3] = {nullptr, nullptr, nullptr};
   float2* fine = nullptr;
   float2* kbuf = nullptr;  // ntrans x M residual scratch for dc
+  std::vector<void*> retired;  // arrays that gbn_plan_reserve replaced
   unsigned* fmax = nullptr;  // ntrans: largest fine cell of each transform (2D tensor-core interp)
   int64_t kbuf_cap = 0;
 
@@ -237,6 +238,7 @@ struct gbn_plan_s {
     dev_free(fine);
     dev_free(kbuf);
     dev_free(fmax);
+    for (void* q : retired) dev_free(q);
     dev_free(tw256);
     dev_free(tw512);
     free_points();
@@ -1165,6 +1167,33 @@ int gbn_plan_tune(gbn_plan p, const int* bins, int interp_method, int maxsub_cap
       p->maxsub_cap = maxsub_cap;
       p->M = -1;
     }
+  });
+}
+
+int gbn_plan_reserve(gbn_plan p, int ntrans) {
+  return guarded(p, [&] {
+    if (ntrans < 1) fail(GBN_ERR_ARG, "ntrans must be >= 1");
+    if (ntrans <= p->ntrans) return;
+    // work in flight and captured graphs may hold the old arrays: they live as
+    // long as the plan
+    p->retired.reserve(p->retired.size() + 2);
+    int64_t added = 0;
+    float2* const fine = dev_alloc<float2>((size_t)ntrans * p->g.G, added, "fine grid");
+    if (p->fmax) {
+      unsigned* fmax = nullptr;
+      try {
+        fmax = dev_alloc<unsigned>(ntrans, added, "fine-grid maxima");
+      } catch (...) {
+        dev_free(fine);
+        throw;
+      }
+      p->retired.push_back(p->fmax);
+      p->fmax = fmax;
+    }
+    p->retired.push_back(p->fine);
+    p->fine = fine;
+    p->bytes += added;
+    p->ntrans = ntrans;
   });
 }
 

@@ -112,12 +112,19 @@ class MRIGB300(_Base):
         self.dtype = np.float32
         self._set_samples(samples)
         G = fine_cells(self.shape, self.eps, self.upsampfac)
-        cap = max(1, int(fine_budget_bytes // (8 * G)))
-        self._ntrans = max(1, min(max(n_batchs * n_coils, n_trans), cap, 64))
+        self._cap = max(1, min(int(fine_budget_bytes // (8 * G)), 64))  # transforms of a pass
+        self._ntrans = max(1, min(max(n_batchs * n_coils, n_trans), self._cap))
         self._plan = NufftPlan(self.shape, self.eps, self.upsampfac, self._ntrans, device=self.device.index)
         self._plan.setpts(self._samples_d)
         self.compute_density(density)
         self.compute_smaps(smaps)
+
+    def _reserve(self, transforms):
+        """Passes of up to ``transforms``, within the fine-grid budget."""
+        n = min(int(transforms), self._cap)
+        if n > self._ntrans:
+            self._plan.reserve(n)
+            self._ntrans = n
 
     # ----------------------------------------------------------------- state
     def _set_samples(self, samples, unsafe=False):

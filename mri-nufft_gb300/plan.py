@@ -95,6 +95,11 @@ class NufftPlan:
         if self._coords is not None and (bins is not None or maxsub_cap):
             self._reset_points()
 
+    def reserve(self, ntrans):
+        """Raise the transforms of a pass to at least ``ntrans``."""
+        _lib.check(self.lib.gbn_plan_reserve(self._h, int(ntrans)), "gbn_plan_reserve")
+        self.ntrans = max(self.ntrans, int(ntrans))
+
     def _reset_points(self):
         cols = self._coords
         M = self.n_samples

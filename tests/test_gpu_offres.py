@@ -67,3 +67,22 @@ def test_adjointness_dc_and_lipschitz(gpu_pkg):
     assert isinstance(cor.op(xt), torch.Tensor)
     L = cor.get_lipschitz_cst(20)
     assert np.isfinite(L) and L > 0
+
+
+def test_passes_grow_with_the_interpolators(gpu_pkg):
+    """The plan of a 2D operator takes up to 64 effective coils a pass once it is
+    corrected; the uncorrected operator gives the same values as before."""
+    rng = np.random.default_rng(5)
+    shape, C, L, M = (32, 24), 3, 25, 700
+    k = rng.uniform(-0.5, 0.5, (M, 2)).astype(np.float32)
+    cpx = lambda *s: (rng.standard_normal(s) + 1j * rng.standard_normal(s)).astype(np.complex64)
+    smaps, x, y = cpx(C, *shape), cpx(1, 1, *shape), cpx(1, C, M)
+    op = gpu_pkg.MRIGB300(k, shape, n_coils=C, smaps=smaps, squeeze_dims=False)
+    before = op.op(x), op.adj_op(y)
+    B, Cl = cpx(M, L), cpx(L, *shape)
+    off = gpu_pkg.MRIFourierCorrectedGB300(op, interpolator=(B, Cl))
+    assert op.plan.ntrans == 64
+    ref = sum(B[:, i] * op.op(x * Cl[i])[0] for i in range(L))
+    assert np.linalg.norm(off.op(x)[0] - ref) < 1e-5 * np.linalg.norm(ref)
+    for a, b in zip(before, (op.op(x), op.adj_op(y))):
+        assert np.linalg.norm(a - b) < 1e-5 * np.linalg.norm(a)
