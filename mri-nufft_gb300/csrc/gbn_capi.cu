@@ -20,8 +20,8 @@
 #include <vector>
 
 #include "gbn_batch.cuh"
-#include "gbn_fft256.cuh"
-#include "gbn_fft512.cuh"
+#include "gbn_fft2d.cuh"
+#include "gbn_fft3d.cuh"
 #include "gbn_internal.cuh"
 #include "gbn_passes.cuh"
 #include "gbn_sort.cuh"
@@ -203,14 +203,11 @@ struct gbn_plan_s {
   bool prune = false;
   cufftHandle pl_lo = 0, pl_span = 0, pl_hi = 0, pl_x = 0;
 
-  // 256^3 fine grids: the fused pruned line transforms of gbn_fft256.cu
-  // replace the pad pass, cuFFT and the crop pass of op / adj / dc
-  bool fft256 = false;
-  float2* tw256 = nullptr;  // W256^k table
-  // 512^2 fine grids (2D): the same with the 512-point line transforms of
-  // gbn_fft512.cu
-  bool fft512 = false;
-  float2* tw512 = nullptr;  // W512^(b k1) table
+  // fine grids whose axes have fused pruned line transforms (gbn_fft2d.cu,
+  // gbn_fft3d.cu), which replace the pad pass, cuFFT and the crop pass
+  bool fft2d = false, fft3d = false;
+  float2* tw_axis[3] = {nullptr, nullptr, nullptr};
+  Twiddles twiddles() const { return Twiddles{{tw_axis[0], tw_axis[1], tw_axis[2]}}; }
 
   // per-stage CUDA-event timing (gbn_profile) and kernel launch count
   bool prof = false;
@@ -239,8 +236,7 @@ struct gbn_plan_s {
     dev_free(kbuf);
     dev_free(fmax);
     for (void* q : retired) dev_free(q);
-    dev_free(tw256);
-    dev_free(tw512);
+    for (float2* t : tw_axis) dev_free(t);
     free_points();
     free_bins();
     dev_free(sb.d_total);
@@ -448,7 +444,7 @@ void setup_tc(gbn_plan p) {
   ck(tc_spread_prepare(), "spread kernel attributes");
   ck(tc_interp_prepare(), "interp kernel attributes");
   tc_error_flag();
-  if (!p->fmax && p->fft512) p->fmax = dev_alloc<unsigned>(p->ntrans, p->bytes, "fine-grid maxima");
+  if (!p->fmax && p->fft2d) p->fmax = dev_alloc<unsigned>(p->ntrans, p->bytes, "fine-grid maxima");
 }
 
 void require_points(gbn_plan p) {
@@ -459,10 +455,15 @@ void require_points(gbn_plan p) {
 }
 
 // Tensor-core interpolation: 2D plans with its tables whose transforms leave the
-// largest fine cell, from 25 transforms on.  Radial 256 x 512 samples, 512^2 grids,
-// interp + transforms against the gather kernel: 64 transforms 320 / 457 us, 32
-// 198 / 235, 24 173 / 185 (spiral 176 / 176), 16 136 / 131.
-bool use_tc_interp(gbn_plan p, int ntr) { return p->tc && p->fft512 && p->g.method_interp == 0 && ntr > 24; }
+// largest fine cell, from 25 transforms on; up to 48 only with a sample for every
+// 4 cells, as it loads each cell of a tile once for all samples of it.  Radial
+// 256 x 512 samples, interp + transforms against the gather kernel: 512^2 cells 64
+// transforms 318 / 454 us, 32 195 / 235, 24 173 / 185 (spiral 176 / 176), 16 136 /
+// 131; 256^2 cells 32 transforms 103 / 156; 640^2 330 / 346; 768^2 (0.22 samples
+// per cell) 464 / 439, with 64 transforms 784 / 820.
+bool use_tc_interp(gbn_plan p, int ntr) {
+  return p->tc && p->fft2d && p->g.method_interp == 0 && ntr > 24 && (ntr > 48 || 4 * p->M >= p->g.G);
+}
 
 void run_interp(gbn_plan p, const InterpArgs& a, cudaStream_t st) {
   if (a.s.nsub == 0) return;
@@ -504,20 +505,20 @@ void run_crop(gbn_plan p, const CropArgs& a, cudaStream_t st) {
   ck(launch_crop(a, st), "crop pass");
   p->launches++;
 }
-// op: pad + forward transform (fused line transforms on 256^3 and 512^2 grids);
+// op: pad + forward transform (fused line transforms where the axes have them);
 // before an interpolation that scales by it, also the largest cell of every grid
 void run_pad_fft(gbn_plan p, const PadArgs& pa, int isign, cudaStream_t st, bool interp_next = false) {
   PadArgs a = pa;
   a.fmax = interp_next && use_tc_interp(p, a.ntr) ? p->fmax : nullptr;
-  if (p->fft512) {
+  if (p->fft2d) {
     Span span(p, GBN_STAGE_FFT, st);
-    ck(launch_fft512_op(a, p->tw512, isign, st), "fused pad + transform");
+    ck(launch_fft2d_op(a, p->twiddles(), isign, st), "fused pad + transform");
     p->launches += 2;
     return;
   }
-  if (p->fft256) {
+  if (p->fft3d) {
     Span span(p, GBN_STAGE_FFT, st);
-    ck(launch_fft256_op(a, p->tw256, isign, st), "fused pad + transform");
+    ck(launch_fft3d_op(a, p->twiddles(), isign, st), "fused pad + transform");
     p->launches += 3;
     return;
   }
@@ -526,16 +527,16 @@ void run_pad_fft(gbn_plan p, const PadArgs& pa, int isign, cudaStream_t st, bool
 }
 // adjoint: inverse transform + crop
 void run_fft_crop(gbn_plan p, const CropArgs& a, int isign, cudaStream_t st) {
-  if (p->fft512) {
+  if (p->fft2d) {
     Span span(p, GBN_STAGE_FFT, st);
-    ck(launch_fft512_adj(a, const_cast<float2*>(a.fine), p->tw512, isign, st),
+    ck(launch_fft2d_adj(a, const_cast<float2*>(a.fine), p->twiddles(), isign, st),
        "fused transform + crop");
     p->launches += 2;
     return;
   }
-  if (p->fft256) {
+  if (p->fft3d) {
     Span span(p, GBN_STAGE_FFT, st);
-    ck(launch_fft256_adj(a, p->fine, p->tw256, isign, st), "fused transform + crop");
+    ck(launch_fft3d_adj(a, p->fine, p->twiddles(), isign, st), "fused transform + crop");
     p->launches += 3;
     return;
   }
@@ -780,21 +781,17 @@ int gbn_plan_create(int dim, const int64_t* n_modes, double upsampfac, double ep
       const char* e = std::getenv("GBN_FFT_PRUNE");
       p->prune = dim == 3 && !spread_only && g.nf[0] > g.n[0] && !(e && std::atoi(e) == 0);
       const char* f = std::getenv("GBN_FUSED_FFT");
-      p->fft256 = !spread_only && fft256_fits(g) && !(f && std::atoi(f) == 0);
-      if (p->fft256) {
-        std::vector<float> t = fft256_twiddles();
-        p->tw256 = dev_alloc<float2>(256, p->bytes, "transform twiddles");
-        ck(cudaMemcpy(p->tw256, t.data(), t.size() * sizeof(float), cudaMemcpyHostToDevice),
-           "copy transform twiddles");
-        ck(fft256_prepare(), "transform kernel attributes");
-      }
-      p->fft512 = !spread_only && fft512_fits(g) && !(f && std::atoi(f) == 0);
-      if (p->fft512) {
-        std::vector<float> t = fft512_twiddles();
-        p->tw512 = dev_alloc<float2>(512, p->bytes, "transform twiddles");
-        ck(cudaMemcpy(p->tw512, t.data(), t.size() * sizeof(float), cudaMemcpyHostToDevice),
-           "copy transform twiddles");
-        ck(fft512_prepare(), "transform kernel attributes");
+      const bool fused = !spread_only && !(f && std::atoi(f) == 0);
+      p->fft2d = fused && fft2d_fits(g);
+      p->fft3d = fused && fft3d_fits(g);
+      if (p->fft2d || p->fft3d) {
+        for (int d = 0; d < dim; ++d) {
+          std::vector<float> t = fft_twiddles(g.nf[d]);
+          p->tw_axis[d] = dev_alloc<float2>(g.nf[d], p->bytes, "transform twiddles");
+          ck(cudaMemcpy(p->tw_axis[d], t.data(), t.size() * sizeof(float), cudaMemcpyHostToDevice),
+             "copy transform twiddles");
+        }
+        ck(p->fft2d ? fft2d_prepare(g) : fft3d_prepare(), "transform kernel attributes");
       }
     }
     p->fine = dev_alloc<float2>((size_t)ntrans * g.G, p->bytes, "fine grid");
@@ -1338,15 +1335,15 @@ void toep_apply(gbn_toep t, const void* img, const void* smaps, void* out, int B
                                 accumulate || c0 > 0, sc)
                     : crop_args(p, nullptr, o + (int64_t)c0 * g.Nimg, T, accumulate, sc);
     ca.dec[0] = ca.dec[1] = ca.dec[2] = nullptr;
-    if (p->fft256) {  // the x transforms and the multiply in one pass over the lines
+    if (p->fft3d && g.nf[0] == 256) {  // the x transforms and the multiply in one pass over the lines
       Span span(p, GBN_STAGE_FFT, st);
-      ck(launch_fft256_gram(pa, ca, t->K, p->tw256, st), "fused Toeplitz Gram");
+      ck(launch_fft3d_gram(pa, ca, t->K, p->twiddles(), st), "fused Toeplitz Gram");
       p->launches += 5;
       return;
     }
-    if (p->fft512) {
+    if (p->fft2d && g.nf[0] == 512) {
       Span span(p, GBN_STAGE_FFT, st);
-      ck(launch_fft512_gram(pa, ca, t->K, p->tw512, st), "fused Toeplitz Gram");
+      ck(launch_fft2d_gram(pa, ca, t->K, p->twiddles(), st), "fused Toeplitz Gram");
       p->launches += 3;
       return;
     }

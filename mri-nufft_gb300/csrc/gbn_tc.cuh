@@ -159,10 +159,10 @@ __device__ __forceinline__ void red_add4(float2* p, float4 v) {
 }
 
 // Power-of-two scale 2^-e that brings values of magnitude up to `m` to below 2
-// (m = 0: e = 0).  e is held to [-96, 126] so that 2^-e and 2^(e - 28) are
+// (m = 0 or infinite: e = 0).  e is held to [-96, 126] so that 2^-e and 2^(e - 28) are
 // normal numbers; at 126 values stay below 4.
 __device__ __forceinline__ int scale_exp(float m) {
-  if (!(m > 0.f)) return 0;
+  if (!(m > 0.f) || m > 3.402823466e38f) return 0;
   const int e = (int)(__float_as_uint(m) >> 23) - 127;
   return e < -96 ? -96 : e > 126 ? 126 : e;
 }

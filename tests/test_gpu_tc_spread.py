@@ -78,3 +78,11 @@ def test_interp_against_fp32_gather(gpu_pkg, monkeypatch, shape, M, C, eps):
     for c in range(C):
         assert rel_l2(out[0][0][0, c], out[1][0][0, c]) < BOUND, c
         assert rel_l2(out[0][1][0, c], out[1][1][0, c]) < 2 * BOUND, c
+
+
+@pytest.mark.parametrize("shape,M,C", [((128, 128), 20000, 27), ((128, 128), 16384, 25), ((128, 128), 16383, 25),
+                                       ((127, 190), 30000, 48), ((320, 128), 900, 49), ((192, 320), 61440, 33)])
+def test_interp_on_other_grids(gpu_pkg, monkeypatch, shape, M, C):
+    """The same two on the other grids with fused transforms, on both sides of the
+    dispatch's lines: 24 transforms, 48, and a sample for every 4 cells."""
+    test_interp_against_fp32_gather(gpu_pkg, monkeypatch, shape, M, C, 1e-6)
