@@ -146,6 +146,11 @@ int gbn_dc(gbn_plan plan, const void* img, const void* obs, const float* density
  * (finufft.py:233-239, cufinufft.py:1319-1325).
  */
 int gbn_pipe(gbn_plan plan, void* w, int iters, float scale2, gbn_stream stream);
+/* The same for real weights (M floats, in place), on half the bytes.  Plans that
+ * have the kernels for it (3D, widths 4 to 7, default bins) answer
+ * gbn_pipe_real_ok with 1; others refuse with GBN_ERR_ARG. */
+int gbn_pipe_real_ok(gbn_plan plan);
+int gbn_pipe_real(gbn_plan plan, float* w, int iters, float scale2, gbn_stream stream);
 
 /*
  * Trajectory gradient of the forward operator, replacing

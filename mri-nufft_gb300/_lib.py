@@ -49,6 +49,8 @@ SIGNATURES = {
     "gbn_adj": (_c_int, [_vp, _vp, _vp, _vp, _vp, _c_int, _c_int, _c_flt, _c_int, _vp]),
     "gbn_dc": (_c_int, [_vp, _vp, _vp, _vp, _vp, _vp, _c_int, _c_int, _c_flt, _vp]),
     "gbn_pipe": (_c_int, [_vp, _vp, _c_int, _c_flt, _vp]),
+    "gbn_pipe_real_ok": (_c_int, [_vp]),
+    "gbn_pipe_real": (_c_int, [_vp, _vp, _c_int, _c_flt, _vp]),
     "gbn_grad_traj_op": (_c_int, [_vp, _vp, _vp, _vp, _vp, _c_int, _c_int, _c_flt, _vp]),
     "gbn_grad_traj_adj": (_c_int, [_vp, _vp, _vp, _vp, _vp, _c_int, _c_int, _c_flt, _vp]),
     "gbn_batch_create": (_c_int, [_c_int, ctypes.POINTER(_vp), ctypes.POINTER(_vp)]),

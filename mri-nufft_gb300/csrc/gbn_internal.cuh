@@ -195,6 +195,10 @@ cudaError_t launch_spread2d(const SpreadArgs& a, cudaStream_t st);
 cudaError_t launch_spread3d(const SpreadArgs& a, cudaStream_t st);
 // column-streaming spreaders; a.s is the column-chunk table
 cudaError_t launch_spread_stream3d(const SpreadArgs& a, cudaStream_t st);
+// one transform with real strengths, cells and values (widths 4 to 7, 8 x 8 bins;
+// the arguments' in, fine and out point to floats); interp: INTERP_PIPE
+cudaError_t launch_spread_real3d(const SpreadArgs& a, cudaStream_t st);
+cudaError_t launch_interp_real3d(const InterpArgs& a, cudaStream_t st);
 cudaError_t launch_spread_stream2d(const SpreadArgs& a, cudaStream_t st);
 cudaError_t launch_grad2d(const GradArgs& a, cudaStream_t st);
 cudaError_t launch_grad3d(const GradArgs& a, cudaStream_t st);

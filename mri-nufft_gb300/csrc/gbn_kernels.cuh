@@ -164,17 +164,21 @@ __device__ __forceinline__ void load_tiles(float2* tile, const float2* __restric
 }
 
 // Asynchronous global -> shared copies of one tile (cp.async, 8 bytes per
-// cell), with the same row / column split as load_tiles.
-__device__ __forceinline__ void cp_async8(float2* dst, const float2* src) {
+// complex cell, 4 per real one), with the same row / column split as load_tiles.
+__device__ __forceinline__ void cp_async_cell(float2* dst, const float2* src) {
   unsigned d = (unsigned)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_cell(float* dst, const float* src) {  // one real cell
+  unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(d), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
-template <int DIM>
-__device__ __forceinline__ void load_tile_async(float2* tile, const float2* __restrict__ fine,
+template <int DIM, class E>
+__device__ __forceinline__ void load_tile_async(E* tile, const E* __restrict__ fine,
                                                 const Geom& g, const int* o, const int* rowoff) {
   const int last = DIM - 1;
   const int pl = g.pd[last];
@@ -187,7 +191,7 @@ __device__ __forceinline__ void load_tile_async(float2* tile, const float2* __re
   const int mc = wrap_idx(o[last] + col, g.nf[last]);
   if (rowoff) {
     for (int r = threadIdx.x / seg; r < nrows; r += step)
-      cp_async8(tile + r * pl + col, fine + rowoff[r] + mc);
+      cp_async_cell(tile + r * pl + col, fine + rowoff[r] + mc);
     return;
   }
   for (int r = threadIdx.x / seg; r < nrows; r += step) {
@@ -200,7 +204,7 @@ __device__ __forceinline__ void load_tile_async(float2* tile, const float2* __re
       rowbase = ((int64_t)wrap_idx(o[0] + i0, g.nf[0]) * g.nf[1] + wrap_idx(o[1] + i1, g.nf[1])) *
                 g.nf[2];
     }
-    cp_async8(tile + r * pl + col, fine + rowbase + mc);
+    cp_async_cell(tile + r * pl + col, fine + rowbase + mc);
   }
 }
 
@@ -260,6 +264,26 @@ GBN_UNROLL
   }
 }
 
+// The same over a tile of real cells (3D, one transform).
+template <int W>
+__device__ __forceinline__ float interp_footprint_real(const float* cur, const Geom& g, const float* w0,
+                                                       const float* w1, const float* w2, int l0, int l1,
+                                                       int l2) {
+  float acc = 0.f;
+#pragma unroll
+  for (int t0 = 0; t0 < W; ++t0) {
+#pragma unroll
+    for (int t1 = 0; t1 < W; ++t1) {
+      const float* row = cur + ((l0 + t0) * g.pd[1] + (l1 + t1)) * g.pd[2] + l2;
+      float sv = 0.f;
+#pragma unroll
+      for (int t2 = 0; t2 < W; ++t2) sv = fmaf(w2[t2], row[t2], sv);
+      acc = fmaf(w0[t0] * w1[t1], sv, acc);
+    }
+  }
+  return acc;
+}
+
 // Interp epilogue of one sample (original index j) for transforms c0 .. c0+nc-1.
 template <int CG>
 __device__ __forceinline__ void interp_store(const InterpArgs& a, int j, int c0, int nc,
@@ -294,11 +318,15 @@ GBN_UNROLL
 // One CTA per subproblem.  When the subproblem has at most one sample per
 // thread, each thread evaluates its sample's kernel weights once and keeps
 // them in registers for every transform pass; larger subproblems evaluate
-// them per pass.
-template <int DIM, int W, int CG>
+// them per pass.  Real cells (E = float): the 3D pipe iteration, whose out is w,
+// one float a sample.
+template <int DIM, int W, int CG, class E = float2>
 __device__ __forceinline__ void interp_body(const InterpArgs& a, const int sub) {
   constexpr int WM = WidthTraits<W>::WM;
-  extern __shared__ float2 tile[];
+  constexpr bool REAL = sizeof(E) == sizeof(float);
+  constexpr int L = REAL ? 32 : 16;  // lanes whose loads are served together
+  extern __shared__ float2 s_tile[];
+  E* const tile = reinterpret_cast<E*>(s_tile);
   const Geom& g = a.g;
   const int b = a.s.sub_bin[sub];
   const int p0 = a.s.sub_start[sub];
@@ -322,12 +350,13 @@ __device__ __forceinline__ void interp_body(const InterpArgs& a, const int sub) 
     // one broadcast.  The samples are sorted by (origin mod 16, origin) and
     // the runs of equal origins are dealt round-robin to the half-warps; in
     // a model of the 3D kooshball this takes the wavefronts per half-warp
-    // load from 2.0 (sort order) to 1.29 (ideal 1).
-    __shared__ int s_hist[16];
+    // load from 2.0 (sort order) to 1.29 (ideal 1).  Real cells: whole warps and
+    // residues mod 32.
+    __shared__ int s_hist[L];
     __shared__ int s_slot[GBN_THREADS];
     __shared__ int s_key[GBN_THREADS];   // origin cell, by residue bucket
     __shared__ int s_who[GBN_THREADS];   // sample index, by residue bucket
-    if (threadIdx.x < 16) s_hist[threadIdx.x] = 0;
+    if (threadIdx.x < L) s_hist[threadIdx.x] = 0;
     s_slot[threadIdx.x] = -1;
     __syncthreads();
     int r = 0, rank = 0, base = 0;
@@ -337,7 +366,7 @@ __device__ __forceinline__ void interp_body(const InterpArgs& a, const int sub) 
       const int l1 = (int)ceilf(a.s.u[1][pos] - g.halfw) - o[1];
       base = l0 * g.pd[1] + l1;
       if (DIM == 3) base = base * g.pd[2] + (int)ceilf(a.s.u[2][pos] - g.halfw) - o[2];
-      r = base & 15;
+      r = base & (L - 1);
       rank = atomicAdd(&s_hist[r], 1);
     }
     __syncthreads();
@@ -372,7 +401,7 @@ __device__ __forceinline__ void interp_body(const InterpArgs& a, const int sub) 
     __shared__ int s_wcnt[GBN_THREADS / 32];
     __shared__ int s_hfill[16], s_fpre[17], s_opre[17];
     int* const s_rstart = s_key;  // run start positions (written after the key reads)
-    const int nh = (cnt + 15) >> 4;
+    const int nh = (cnt + L - 1) / L;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int p = threadIdx.x;
     const bool in = p < cnt;
@@ -403,8 +432,8 @@ __device__ __forceinline__ void interp_body(const InterpArgs& a, const int sub) 
         s_fpre[h] = f;
         s_opre[h] = ov;
         const int fl = s_hfill[h];
-        f += fl < 16 ? 16 - fl : 0;
-        ov += fl > 16 ? fl - 16 : 0;
+        f += fl < L ? L - fl : 0;
+        ov += fl > L ? fl - L : 0;
       }
       s_fpre[nh] = f;
       s_opre[nh] = ov;
@@ -413,13 +442,13 @@ __device__ __forceinline__ void interp_body(const InterpArgs& a, const int sub) 
     if (in) {
       const int h = run % nh;
       const int ln = s_rpos[run] + (p - s_rstart[run]);
-      if (ln < 16) {
-        s_slot[h * 16 + ln] = s_who[p];
+      if (ln < L) {
+        s_slot[h * L + ln] = s_who[p];
       } else {  // k-th overflow sample -> k-th free lane
-        const int k = s_opre[h] + ln - 16;
+        const int k = s_opre[h] + ln - L;
         int hh = 0;
         while (hh + 1 < nh && s_fpre[hh + 1] <= k) ++hh;
-        s_slot[hh * 16 + s_hfill[hh] + (k - s_fpre[hh])] = s_who[p];
+        s_slot[hh * L + s_hfill[hh] + (k - s_fpre[hh])] = s_who[p];
       }
     }
     __syncthreads();
@@ -434,6 +463,26 @@ __device__ __forceinline__ void interp_body(const InterpArgs& a, const int sub) 
   }
   __syncthreads();
 
+  if constexpr (REAL) {
+    load_tile_async<DIM>(tile, reinterpret_cast<const float*>(a.fine), g, o, rowoff);
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+    float* const out = reinterpret_cast<float*>(a.out);
+    if (cached) {
+      if (cj >= 0)
+        out[cj] /= a.scale * fabsf(interp_footprint_real<W>(tile, g, cw0, cw1, cw2, cl0, cl1, cl2));
+      return;
+    }
+    for (int s = threadIdx.x; s < cnt; s += blockDim.x) {
+      const int pos = p0 + s;
+      const int l0 = weights_rt<W>(a.s.u[0][pos], g, cw0) - o[0];
+      const int l1 = weights_rt<W>(a.s.u[1][pos], g, cw1) - o[1];
+      const int l2 = weights_rt<W>(a.s.u[2][pos], g, cw2) - o[2];
+      out[a.s.perm[pos]] /= a.scale * fabsf(interp_footprint_real<W>(tile, g, cw0, cw1, cw2, l0, l1, l2));
+    }
+    return;
+  } else {
   for (int c0 = 0; c0 < a.ntr; c0 += CG) {
     const int nc = imin(CG, a.ntr - c0);
     if (rowoff) {
@@ -465,6 +514,7 @@ __device__ __forceinline__ void interp_body(const InterpArgs& a, const int sub) 
       }
     }
     __syncthreads();
+  }
   }
 }
 

@@ -564,7 +564,7 @@ class MRIGB300(_Base):
         grid = NufftPlan(volume_shape, eps=eps, upsampfac=float(osf), ntrans=1, spread_only=True,
                          device=dev.index)
         grid.setpts(s)
-        w = torch.ones(s.shape[0], dtype=torch.complex64, device=dev)
+        w = torch.ones(s.shape[0], dtype=torch.float32 if grid.real_pipe else torch.complex64, device=dev)
         nf = np.sqrt(np.prod(volume_shape) * 2 ** len(volume_shape))
         grid.pipe(w, max_iter, 1.0 / (nf * nf))
         if normalize:

@@ -164,7 +164,16 @@ class NufftPlan:
         )
         return out
 
+    @property
+    def real_pipe(self):
+        """Whether :meth:`pipe` takes real (float32) weights too."""
+        return bool(self.lib.gbn_pipe_real_ok(self._h))
+
     def pipe(self, w, iters, scale2):
+        if w.dtype == torch.float32:
+            _lib.check(self.lib.gbn_pipe_real(self._h, _ptr(w), int(iters), float(scale2), self.stream),
+                       "gbn_pipe_real")
+            return w
         _lib.check(self.lib.gbn_pipe(self._h, _ptr(w), int(iters), float(scale2), self.stream),
                    "gbn_pipe")
         return w
