@@ -694,14 +694,7 @@ int gbn_plan_create(int dim, const int64_t* n_modes, double upsampfac, double ep
     // 2D: 19-cell x bins (with w <= 7 the padded column is at most 25 rows,
     // two overlapping 16-row halves of a warp in the streaming spreader)
     int binsz2[2] = {19, 32};
-    // 3D: the z extent gives the interp's padded tile an odd row pitch (15 or, for the
-    // smaller tensor-core cross-sections, 31 cells), so that the rows of a footprint
-    // start on different banks and a tile's cells serve more samples.  2.1 M samples,
-    // 128^3 images, interp: 1 coil z = 8 308 us, 9 292 (64^3 178 / 174), longer ones
-    // slower there; 16 coils z = 16 4.66 ms, 24 4.33, 25 4.38, 26 (pitch 32) 5.52;
-    // 3 coils of 97 x 110 x 75 313 / 270 / 259 / 332 us; 96^3 w = 5 z = 16 504, 27
-    // 472, 28 (pitch 32) 618.
-    int binsz3[3] = {8, 8, w <= 7 ? 16 - w : 8};
+    int binsz3[3] = {8, 8, 8};
     const char* sp = std::getenv("GBN_SPREAD");
     const bool want_tc = sp && std::strcmp(sp, "mma") == 0;
     // Plans of several transforms: the tiles of the tensor-core spreaders.
@@ -712,7 +705,12 @@ int gbn_plan_create(int dim, const int64_t* n_modes, double upsampfac, double ep
     if (!spread_only && w <= 7 && (want_tc || (!sp && ntrans >= 2))) {
       binsz2[0] = tc_bin(2, w);
       binsz3[0] = binsz3[1] = tc_bin(3, w);
-      binsz3[2] = 32 - w;
+      // z: the interp's padded tiles; longer ones serve more samples a cell, a pitch
+      // of 32 cells puts every row on the same banks, and an even extent and pitch
+      // load two cells at a time.  Interp of 16 coils, 2.1 M samples: z = 16 4.66 ms,
+      // 22 3.74, 24 3.60, 25 (pitch 31, single cells) 4.38, 26 (pitch 32) 5.52;
+      // 3 coils of 97 x 110 x 75 313 / 237 / 234 / 262 / 332 us.
+      binsz3[2] = (31 - w) & ~1;
     }
     // tuning overrides: GBN_BINS2="b0,b1", GBN_BINS3="b0,b1,b2", GBN_INTERP_CG=1|2|4
     if (const char* e = std::getenv(dim == 2 ? "GBN_BINS2" : "GBN_BINS3")) {
@@ -764,7 +762,7 @@ int gbn_plan_create(int dim, const int64_t* n_modes, double upsampfac, double ep
         g.bs[d] = bs;
         g.nkey[d] = (int)nf + g.koff - w / 2;
         g.nb[d] = (g.nkey[d] + bs - 1) / bs;
-        g.pd[d] = bs + w - 1;
+        g.pd[d] = d == 2 ? (bs + w) & ~1 : bs + w - 1;  // 3D tile rows: even (pairs of cells)
         g.uscale[d] = (float)((double)nf / (2.0 * M_PI));
       } else {
         g.n[d] = g.nf[d] = g.bs[d] = g.nb[d] = g.pd[d] = g.nkey[d] = 1;
@@ -1190,7 +1188,7 @@ int gbn_plan_tune(gbn_plan p, const int* bins, int interp_method, int maxsub_cap
         if (bins[d] < 1 || bins[d] > 64) fail(GBN_ERR_ARG, "bin sizes must be in [1, 64]");
         t.bs[d] = bins[d] > g.nf[d] ? g.nf[d] : bins[d];
         t.nb[d] = (g.nkey[d] + t.bs[d] - 1) / t.bs[d];
-        t.pd[d] = t.bs[d] + g.w - 1;
+        t.pd[d] = d == 2 ? (t.bs[d] + g.w) & ~1 : t.bs[d] + g.w - 1;
       }
       t.tile = t.pd[0] * t.pd[1] * t.pd[2];
       if ((int64_t)t.tile * 8 > kTileSmemBudget) fail(GBN_ERR_ARG, "tile does not fit shared memory");

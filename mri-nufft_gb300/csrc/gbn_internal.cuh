@@ -27,7 +27,7 @@ struct Geom {
   int nf[3];     // fine grid per axis (unused axes = 1)
   int bs[3];     // bin size per axis (unused axes = 1)
   int nb[3];     // number of bins per axis
-  int pd[3];     // padded tile extent per axis = bs + w - 1 (unused axes = 1)
+  int pd[3];     // padded tile extent per axis: bs + w - 1, even along z (unused axes: 1)
   int nkey[3];   // sort keys per axis: a sample's key is its first footprint cell + koff
   int koff;      // floor(w / 2) rounded up to even, so that even-sized bins start on even cells
   int w;         // kernel width in cells
