@@ -259,6 +259,7 @@ struct gbn_plan_s {
     free_bins();
     tc = !spread_only && tc_fit(g);
     stream_spread = tc || stream_fit(g) ? 1 : 0;
+    g.tile2 = tc && g.dim == 2 && g.w == 7 && g.tile <= 640;
     const int last = g.dim - 1;
     ngrp = g.nb[0] * g.nb[1] * g.nb[2];
     ncol = ngrp / g.nb[last];
@@ -455,14 +456,18 @@ void require_points(gbn_plan p) {
 }
 
 // Tensor-core interpolation: 2D plans with its tables whose transforms leave the
-// largest fine cell, from 25 transforms on; up to 48 only with a sample for every
-// 4 cells, as it loads each cell of a tile once for all samples of it.  Radial
-// 256 x 512 samples, interp + transforms against the gather kernel: 512^2 cells 64
-// transforms 318 / 454 us, 32 195 / 235, 24 173 / 185 (spiral 176 / 176), 16 136 /
-// 131; 256^2 cells 32 transforms 103 / 156; 640^2 330 / 346; 768^2 (0.22 samples
-// per cell) 464 / 439, with 64 transforms 784 / 820.
+// largest fine cell, from 25 transforms on.  It loads each cell of a tile once for
+// all samples of it, so it wants samples.  Interp, and what the largest cell costs
+// the transforms, against the tile kernel of w = 7 (us): 2.3 samples a cell, 32
+// transforms 236 / 350; 0.5 (radial, spiral), 64 transforms 144 / 186 and 155 / 177,
+// 48 132 / 145 and 149 / 136, 32 102 / 102 and 103 / 97; 0.22, 64 213 / 198.
+// Against the gather kernel of the other widths' shape (w = 7 measured): 0.5, 64
+// transforms 144 / 281, 32 102 / 140, 24 about 92 / 104 (spiral 95 / 94); 0.22, 32
+// transforms 186 / 161, 64 267 / 304.
 bool use_tc_interp(gbn_plan p, int ntr) {
-  return p->tc && p->fft2d && p->g.method_interp == 0 && ntr > 24 && (ntr > 48 || 4 * p->M >= p->g.G);
+  if (!p->tc || !p->fft2d || p->g.method_interp != 0 || ntr <= 24) return false;
+  if (p->g.tile2) return (ntr > 48 ? 3 : 1) * p->M >= p->g.G;
+  return ntr > 48 || 4 * p->M >= p->g.G;
 }
 
 void run_interp(gbn_plan p, const InterpArgs& a, cudaStream_t st) {
@@ -704,6 +709,9 @@ int gbn_plan_create(int dim, const int64_t* n_modes, double upsampfac, double ep
     // columns would be mostly empty).
     if (!spread_only && w <= 7 && (want_tc || (!sp && ntrans >= 2))) {
       binsz2[0] = tc_bin(2, w);
+      // w = 7 interpolates from tiles: 16 radial transforms on 512^2 cells 58 us, with
+      // y = 16 61, 32 64, 48 74 (a row pitch of 30 cells, short tiles for more CTAs)
+      if (w == 7) binsz2[1] = 24;
       binsz3[0] = binsz3[1] = tc_bin(3, w);
       // z: the interp's padded tiles; longer ones serve more samples a cell, a pitch
       // of 32 cells puts every row on the same banks, and an even extent and pitch
@@ -870,8 +878,10 @@ int gbn_setpts(gbn_plan p, int64_t M, const float* k0, const float* k1, const fl
     const int maxsub_i = [&] {
       if (!p->stream_spread) return maxsub;
       const char* e = std::getenv("GBN_INTERP_MAXSUB");
-      int v = e ? std::atoi(e) : 128;
-      if (v < 32) v = 128;
+      // 2D tiles: 64-thread CTAs (768^2 cells, 16 transforms 73 -> 64 us)
+      const int v0 = p->g.tile2 ? 64 : 128;
+      int v = e ? std::atoi(e) : v0;
+      if (v < 32) v = v0;
       return v < maxsub ? v : maxsub;
     }();
     int64_t subcap = M / maxsub_i + (M < p->ngrp ? M : p->ngrp) + 1;

@@ -46,6 +46,7 @@ struct Geom {
                       // 3: 3D column streaming, 4: 3D bin-tile rows,
                       // 5: 3D quadrant streaming (8 x 8 bins), 6: tensor cores (tc_bins)
   int interp_threads; // CTA size of the tile interp kernel (0: 128)
+  int tile2;          // 2D plans of several transforms, w = 7: interpolate from tiles (4 at a time)
   int spread_cg;      // coils per pass of the streaming spreader (0: automatic)
   int quad_minb;      // resident CTAs per SM of the 4-coil quadrant spreader (0: 3)
   int quad_packed;    // 0: scalar accumulators in the quadrant spreader (default 1: (re, im) pairs)

@@ -191,7 +191,8 @@ __device__ __forceinline__ void load_tile_async(E* tile, const E* __restrict__ f
                                                 const Geom& g, const int* o, const int* rowoff) {
   const int last = DIM - 1;
   const int pl = g.pd[last];
-  if (DIM == 3 && rowoff && !((g.nf[2] | o[2] | pl) & 1) &&
+  const int nrows = DIM == 2 ? g.pd[0] : g.pd[0] * g.pd[1];
+  if (rowoff && !((g.nf[last] | o[last] | pl) & 1) &&
       reinterpret_cast<size_t>(fine) % (2 * sizeof(E)) == 0) {
     // Even grids, origins and pitches (and a grid of the caller's that starts on a
     // pair): two cells a copy (a pair never wraps).  The
@@ -201,15 +202,14 @@ __device__ __forceinline__ void load_tile_async(E* tile, const E* __restrict__ f
     while (2 * sg < pl) sg <<= 1;
     const int cp = 2 * (threadIdx.x & (sg - 1));
     if (cp >= pl) return;
-    const int m = wrap_idx(o[2] + cp, g.nf[2]);
-    const int rows = g.pd[0] * g.pd[1], st = blockDim.x / sg;
-    for (int r = threadIdx.x / sg; r < rows; r += st)
+    const int m = wrap_idx(o[last] + cp, g.nf[last]);
+    const int st = blockDim.x / sg;
+    for (int r = threadIdx.x / sg; r < nrows; r += st)
       cp_async_pair(tile + r * pl + cp, fine + rowoff[r] + m);
     return;
   }
   int seg = 16;
   while (seg < pl) seg <<= 1;
-  const int nrows = DIM == 2 ? g.pd[0] : g.pd[0] * g.pd[1];
   const int col = threadIdx.x & (seg - 1);
   if (col >= pl) return;
   const int step = blockDim.x / seg;
@@ -2086,7 +2086,7 @@ cudaError_t launch_interp_t(const InterpArgs& a, cudaStream_t st) {
   if (e != cudaSuccess) return e;
   // 128-thread CTAs: subproblems average fewer samples than 256, and smaller
   // CTAs wait less at the per-coil tile barriers (measured 4 % faster in 3D)
-  const int threads = a.g.interp_threads == 64 ? 64 : kInterpThreads;
+  const int threads = a.g.interp_threads == 64 || (DIM == 2 && a.g.tile2) ? 64 : kInterpThreads;
   k<<<a.s.nsub, threads, smem, st>>>(a);
   return cudaGetLastError();
 }
@@ -2233,6 +2233,15 @@ inline cudaError_t launch_interp_twc(const InterpArgs& a, cudaStream_t st) {
 
 template <int DIM>
 cudaError_t dispatch_interp(const InterpArgs& a, cudaStream_t st) {
+  if constexpr (DIM == 2) {
+    // 4 tiles at a time, whose cells serve all samples on them: 8 / 16 / 24 radial
+    // transforms on 512^2 cells (0.5 samples a cell) 43 / 72 / 104 -> 37 / 58 / 80 us
+    // against the warp-cooperative kernel, 2 25 -> 21; 768^2 (0.22) 41 / 71 / 111 ->
+    // 41 / 64 / 87, 3 27 -> 29; 0.1 samples a cell, 16 transforms 25 -> 32
+    if (a.g.tile2 && a.g.method_interp == 0 && a.ntr > 1 &&
+        (a.ntr > 8 ? 6 : 3) * a.s.M >= a.g.G)
+      return a.ntr > 2 ? dispatch_interp_w<2, 4>(a, st) : dispatch_interp_w<2, 2>(a, st);
+  }
   // 2D at w = 7 defaults to the warp-cooperative direct kernel (measured 1.1x
   // the tile kernel with its bank-aware lane order on the 1024-transform
   // stack-of-stars, 2.7x before it); 3D to tiles.  GBN_INTERP=tile forces tiles.

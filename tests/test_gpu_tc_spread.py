@@ -86,3 +86,13 @@ def test_interp_on_other_grids(gpu_pkg, monkeypatch, shape, M, C):
     """The same two on the other grids with fused transforms, on both sides of the
     dispatch's lines: 24 transforms, 48, and a sample for every 4 cells."""
     test_interp_against_fp32_gather(gpu_pkg, monkeypatch, shape, M, C, 1e-6)
+
+
+@pytest.mark.parametrize("shape,M,C", [((128, 128), 21846, 2), ((128, 128), 21845, 3), ((128, 128), 30000, 5),
+                                       ((128, 128), 10923, 9), ((128, 128), 10922, 9), ((100, 90), 36001, 7),
+                                       ((9, 130), 4001, 4), ((128, 128), 65536, 25), ((128, 128), 22000, 49)])
+def test_interp_from_tiles(gpu_pkg, monkeypatch, shape, M, C):
+    """The same two on both sides of the tile kernel's lines (w = 7): samples a cell,
+    transforms (groups of 4 and 2 with remainders), grids without fused transforms,
+    tiles over both ends of the period, the tensor-core kernel of dense samples."""
+    test_interp_against_fp32_gather(gpu_pkg, monkeypatch, shape, M, C, 1e-6)
