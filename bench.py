@@ -295,7 +295,8 @@ def measure_pipe(pkg, samples_d, shape, device, iters=10, reps=5):
     pplan = pkg.NufftPlan(shape, eps=1e-6, upsampfac=2.0, ntrans=1, spread_only=True, device=device)
     pplan.setpts(samples_d)
     nrm2 = float(np.prod(shape) * 2 ** len(shape))
-    w = torch.ones(M, dtype=torch.complex64, device=dev)
+    real = pplan.real_pipe  # as MRIGB300.pipe
+    w = torch.ones(M, dtype=torch.float32 if real else torch.complex64, device=dev)
     pplan.pipe(w, iters, 1.0 / nrm2)
     torch.cuda.synchronize()
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -312,7 +313,7 @@ def measure_pipe(pkg, samples_d, shape, device, iters=10, reps=5):
     info = pplan.info()
     G_t = touched_cells(samples_d, info["nf"], info["width"])
     spread_ms = st["spread"][0] / max(1, st["spread"][1])
-    bytes_spread = 4 * len(shape) * M + 8 * M + 8 * G_t
+    bytes_spread = 4 * len(shape) * M + (4 if real else 8) * (M + G_t)
     t0 = time.perf_counter()
     pkg.MRIGB300.pipe(samples_d, shape, max_iter=iters, device=device)
     torch.cuda.synchronize()

@@ -2242,9 +2242,8 @@ cudaError_t dispatch_interp(const InterpArgs& a, cudaStream_t st) {
         (a.ntr > 8 ? 6 : 3) * a.s.M >= a.g.G)
       return a.ntr > 2 ? dispatch_interp_w<2, 4>(a, st) : dispatch_interp_w<2, 2>(a, st);
   }
-  // 2D at w = 7 defaults to the warp-cooperative direct kernel (measured 1.1x
-  // the tile kernel with its bank-aware lane order on the 1024-transform
-  // stack-of-stars, 2.7x before it); 3D to tiles.  GBN_INTERP=tile forces tiles.
+  // the rest of 2D at w = 7 takes the warp-cooperative direct kernel, 3D tiles;
+  // GBN_INTERP=tile forces tiles
   if (a.g.w == 7 && (a.g.method_interp == 4 || (DIM == 2 && a.g.method_interp == 0)))
     return launch_interp_wc_t<DIM>(a, st);
   if constexpr (DIM == 2) {  // the widths of eps 1e-3 .. 1e-5
