@@ -254,8 +254,16 @@ struct gbn_plan_s {
     bin_bytes = 0;
   }
 
+  // Refuses a geometry whose bins or sort keys are more than the sort's limit.
+  void check_bins(const Geom& t) const {
+    const int64_t cols = t.dim == 2 ? t.nb[0] : (int64_t)t.nb[0] * t.nb[1];
+    if (cols > kMaxBins || cols * t.nkey[t.dim - 1] > kMaxBins)
+      fail(GBN_ERR_ARG, "too many bins for the fine grid");
+  }
+
   // (Re)allocates the per-bin arrays for the current geometry.
   void setup_bins() {
+    check_bins(g);
     free_bins();
     tc = !spread_only && tc_fit(g);
     stream_spread = tc || stream_fit(g) ? 1 : 0;
@@ -1202,10 +1210,11 @@ int gbn_plan_tune(gbn_plan p, const int* bins, int interp_method, int maxsub_cap
       }
       t.tile = t.pd[0] * t.pd[1] * t.pd[2];
       if ((int64_t)t.tile * 8 > kTileSmemBudget) fail(GBN_ERR_ARG, "tile does not fit shared memory");
+      p->check_bins(t);
+      p->M = -1;  // points must be set again
       g = t;
       p->setup_bins();
       setup_tc(p);
-      p->M = -1;  // points must be set again
     }
     if (interp_method >= 0) {
       if (interp_method > 5 || interp_method == 2) fail(GBN_ERR_ARG, "unknown interpolation method");

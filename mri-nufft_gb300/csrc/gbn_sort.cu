@@ -100,7 +100,10 @@ __global__ void group_kernel(int ngroups, int ngz, int K, int nl, const int* __r
 }
 
 // ---------------------------------------------------------------------------
-// Exclusive scan of int arrays (block scan + scan of block sums + add).
+// Exclusive scan of int arrays (block scan + scan of block sums + add).  The
+// sums of the blocks are scanned the same way, so that the length has no limit
+// but its type: one level to 4096 entries, two to 16.7 M, three beyond (the keys
+// of a 1024^3 grid are 17.1 M, of a 750^3 grid in the tensor-core columns as many).
 // ---------------------------------------------------------------------------
 constexpr int kScanThreads = 1024;
 constexpr int kScanItems = 4;
@@ -172,22 +175,25 @@ __global__ void scan_total_kernel(const int* in, const int* out, int n, int* tot
 }
 
 size_t scan_scratch_ints(int n) {
-  int tiles = (n + kScanTile - 1) / kScanTile;
-  return (size_t)2 * (tiles + 1) + 8;
+  const int tiles = (n - 1) / kScanTile + 1;
+  return (size_t)2 * (tiles + 1) + 8 + (tiles > 1 ? scan_scratch_ints(tiles) : 0);
+}
+
+static void scan_levels(const int* in, int* out, int n, int* scratch, cudaStream_t st) {
+  const int tiles = (n - 1) / kScanTile + 1;
+  int* sums = scratch;
+  int* sums_scan = scratch + tiles + 1;
+  scan_tiles_kernel<<<tiles, kScanThreads, 0, st>>>(in, out, n, tiles > 1 ? sums : nullptr);
+  if (tiles == 1) return;
+  scan_levels(sums, sums_scan, tiles, scratch + 2 * ((size_t)tiles + 1), st);
+  add_tile_offsets_kernel<<<(n - 1) / 256 + 1, 256, 0, st>>>(out, n, sums_scan);
 }
 
 cudaError_t exclusive_scan(const int* in, int* out, int n, int* scratch, int* total,
                            cudaStream_t st) {
   if (n <= 0) return cudaMemsetAsync(total, 0, sizeof(int), st);
-  int tiles = (n + kScanTile - 1) / kScanTile;
-  if (tiles > kScanTile) return cudaErrorInvalidValue;  // > 16.7 M entries
-  int* sums = scratch;
-  int* sums_scan = scratch + tiles + 1;
-  scan_tiles_kernel<<<tiles, kScanThreads, 0, st>>>(in, out, n, tiles > 1 ? sums : nullptr);
-  if (tiles > 1) {
-    scan_tiles_kernel<<<1, kScanThreads, 0, st>>>(sums, sums_scan, tiles, nullptr);
-    add_tile_offsets_kernel<<<(n + 255) / 256, 256, 0, st>>>(out, n, sums_scan);
-  }
+  if (n > kMaxBins) return cudaErrorInvalidValue;
+  scan_levels(in, out, n, scratch, st);
   scan_total_kernel<<<1, 1, 0, st>>>(in, out, n, total);
   return cudaGetLastError();
 }
@@ -209,7 +215,7 @@ cudaError_t build_group_table(int ngroups, int ngz, int K, int nl, int maxsub,
 cudaError_t sort_points(const Geom& g, int64_t M, const float* const k[3], int maxsub,
                         const SortBuffers& sb, cudaStream_t st, bool subproblems) {
   const int nbins = g.nb[0] * g.nb[1] * g.nb[2];
-  cudaError_t e = cudaMemsetAsync(sb.bin_count, 0, sizeof(int) * nbins, st);
+  cudaError_t e = cudaMemsetAsync(sb.bin_count, 0, sizeof(int) * (size_t)nbins, st);
   if (e != cudaSuccess) return e;
   const float* k2 = g.dim == 3 ? k[2] : k[1];
   if (M > 0) {

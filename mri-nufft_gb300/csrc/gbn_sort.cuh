@@ -32,6 +32,10 @@ struct GroupBuffers {
   int* sub_count;
 };
 
+// Largest number of bins or groups: every index of a block of 4096 entries, and
+// every rounding up to a multiple of one, stays an int.
+constexpr int kMaxBins = 2147483647 - 8192;
+
 size_t scan_scratch_ints(int n);
 // Builds gb's subproblem table (chunks of <= maxsub samples per group) from a
 // finished sort; d_total receives the number of subproblems.
