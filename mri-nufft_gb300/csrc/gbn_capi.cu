@@ -1586,6 +1586,7 @@ struct FftGroup {
 
 struct gbn_batch_s {
   std::vector<gbn_plan> plans;
+  std::vector<int> slots;  // fine grids of each instance in its pool: a plan's passes may grow later
   std::vector<BatchInst> h_inst;
   std::vector<FftGroup> groups;
   BatchInst* d_inst = nullptr;
@@ -1632,6 +1633,7 @@ int gbn_batch_create(int n, const gbn_plan* plans, gbn_batch* out) {
       if (plans[0]->g.w != p->g.w) fail(GBN_ERR_ARG, "plans of a batch must share the kernel width");
       rows = rows && rows_fit(p->g);
       b->plans.push_back(p);
+      b->slots.push_back(p->ntrans);
       BatchInst bi{};
       bi.g = p->g;
       bi.s = p->sorted();
@@ -1665,7 +1667,7 @@ int gbn_batch_create(int n, const gbn_plan* plans, gbn_batch* out) {
         b->groups.push_back(gr);
         gi = (int)b->groups.size() - 1;
       }
-      b->groups[gi].slots += p->ntrans;
+      b->groups[gi].slots += b->slots[i];
     }
     for (auto& gr : b->groups) {
       gr.pool = dev_alloc<float2>((size_t)gr.slots * gr.G, tmp, "batch fine-grid pool");
@@ -1682,7 +1684,7 @@ int gbn_batch_create(int n, const gbn_plan* plans, gbn_batch* out) {
           FftGroup& gr = b->groups[k];
           if (gr.nf[0] == p->g.nf[0] && gr.nf[1] == p->g.nf[1] && gr.nf[2] == p->g.nf[2]) {
             b->h_inst[i].fine = gr.pool + (int64_t)used[k] * gr.G;
-            used[k] += p->ntrans;
+            used[k] += b->slots[i];
             break;
           }
         }
@@ -1738,8 +1740,9 @@ int gbn_batch_bind(gbn_batch b, void* const* imgs, const void* const* smaps, voi
     for (size_t i = 0; i < b->plans.size(); ++i) {
       gbn_plan p = b->plans[i];
       BatchInst& bi = b->h_inst[i];
-      if (n_coils[i] < 1 || n_coils[i] > p->ntrans)
-        fail(GBN_ERR_ARG, "instance " + std::to_string(i) + ": n_coils must be in [1, plan ntrans]");
+      if (n_coils[i] < 1 || n_coils[i] > b->slots[i])
+        fail(GBN_ERR_ARG, "instance " + std::to_string(i) +
+                              ": n_coils must be in [1, ntrans of the plan when the batch was made]");
       if (!imgs[i] || (!ksps[i] && p->M > 0)) fail(GBN_ERR_ARG, "null buffer in batch bind");
       bi.img = static_cast<float2*>(imgs[i]);
       bi.smaps = smaps ? static_cast<const float2*>(smaps[i]) : nullptr;
