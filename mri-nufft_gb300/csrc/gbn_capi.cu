@@ -150,7 +150,8 @@ void gbn::set_last_error(const char* msg) { g_err = msg; }
 
 struct gbn_plan_s {
   Geom g{};
-  int ntrans = 1;
+  int ntrans = 1;   // transforms of a pass
+  int ntrans0 = 1;  // as it was created (gbn_plan_reserve raises ntrans)
   int spread_only = 0;
   int device = 0;
   int nsm = 152;
@@ -160,9 +161,10 @@ struct gbn_plan_s {
   float* dec[3] = {nullptr, nullptr, nullptr};
   float2* fine = nullptr;
   float2* kbuf = nullptr;  // ntrans x M residual scratch for dc
-  std::vector<void*> retired;  // arrays that gbn_plan_reserve replaced
+  std::vector<void*> retired;  // arrays replaced while work or captured graphs may use them
   unsigned* fmax = nullptr;  // ntrans: largest fine cell of each transform (2D tensor-core interp)
   int64_t kbuf_cap = 0;
+  int64_t kbuf_M = 0;      // samples it was last used for
 
   // sort state
   int64_t M = -1, Mcap = 0, subcap = 0;
@@ -685,7 +687,7 @@ int gbn_plan_create(int dim, const int64_t* n_modes, double upsampfac, double ep
     DeviceGuard dg(device);
     p = new gbn_plan_s();
     p->device = device;
-    p->ntrans = ntrans;
+    p->ntrans = p->ntrans0 = ntrans;
     p->spread_only = spread_only ? 1 : 0;
     p->eps = eps;
     p->sigma = upsampfac;
@@ -1037,15 +1039,27 @@ int gbn_dc(gbn_plan p, const void* img, const void* obs, const float* density,
     const float2* s = static_cast<const float2*>(smaps);
     float2* gr = static_cast<float2*>(grad);
     const Geom& g = p->g;
-    int64_t need = (int64_t)p->ntrans * (p->M > 0 ? p->M : 1);
+    // passes of this call, at least those the plan was created for: a plan whose passes
+    // were raised keeps the buffer that work in flight and captured graphs use, and a
+    // longer one for more transforms retires it
+    const int rows = s ? C : B * C;
+    const int64_t need = (int64_t)imin(p->ntrans, rows > p->ntrans0 ? rows : p->ntrans0) * (p->M > 0 ? p->M : 1);
     if (need > p->kbuf_cap) {
-      dev_free(p->kbuf);
-      p->bytes -= p->kbuf_cap * 8;
-      p->kbuf = nullptr;
-      p->kbuf_cap = 0;
-      p->kbuf = dev_alloc<float2>(need, p->bytes, "residual buffer");
+      if (p->kbuf && p->kbuf_M == p->M) {
+        p->retired.reserve(p->retired.size() + 1);
+        float2* const grown = dev_alloc<float2>(need, p->bytes, "residual buffer");
+        p->retired.push_back(p->kbuf);
+        p->kbuf = grown;
+      } else {  // other samples: what was captured with the old ones is void
+        dev_free(p->kbuf);
+        p->bytes -= p->kbuf_cap * 8;
+        p->kbuf = nullptr;
+        p->kbuf_cap = 0;
+        p->kbuf = dev_alloc<float2>(need, p->bytes, "residual buffer");
+      }
       p->kbuf_cap = need;
     }
+    p->kbuf_M = p->M;
     for_each_pass(p, s != nullptr, B, C, [&](int b, int c0, int T) {
       PadArgs pa = s ? pad_args(p, x + (int64_t)b * g.Nimg, s + (int64_t)c0 * g.Nimg, T, 0)
                      : pad_args(p, x + (int64_t)c0 * g.Nimg, nullptr, T, 0);

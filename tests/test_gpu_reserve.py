@@ -28,3 +28,29 @@ def test_batch_keeps_the_slots_it_was_made_with(gpu_pkg):
     bat.coils[0] = 3
     with pytest.raises(ValueError):
         bat._bind()
+
+
+def test_captured_data_consistency_outlives_a_reserve(gpu_pkg):
+    """A captured gradient keeps its residual buffer when the plan's passes grow,
+    and when a later call with more transforms needs a longer one."""
+    C, n, M = 2, 24, 500
+    k = torch.from_numpy(np.random.default_rng(1).uniform(-3, 3, (M, 2)).astype(np.float32)).cuda()
+    plan = gpu_pkg.NufftPlan((n, n), ntrans=C)
+    plan.setpts(k)
+    x, y, out = _cpx(C, n, n), _cpx(C, M), _cpx(C, n, n)
+    plan.dc(x, y, None, None, out, 1, C, 1.0)
+    want = out.clone()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        plan.dc(x, y, None, None, out, 1, C, 1.0)
+    plan.reserve(16)
+    before = plan.device_bytes
+    plan.dc(x, y, None, None, out, 1, C, 1.0)
+    assert plan.device_bytes == before  # the same call needs no longer buffer
+    x2, y2 = _cpx(16, n, n), _cpx(16, M)
+    plan.dc(x2, y2, None, None, torch.empty_like(x2), 1, 16, 1.0)
+    assert plan.device_bytes >= before + 8 * 16 * M
+    out.zero_()
+    graph.replay()
+    assert (torch.linalg.norm(out - want) / torch.linalg.norm(want)).item() < 1e-5
