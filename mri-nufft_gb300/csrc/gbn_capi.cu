@@ -15,6 +15,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <map>
+#include <mutex>
 #include <new>
 #include <string>
 #include <vector>
@@ -153,6 +154,7 @@ struct gbn_plan_s {
   int ntrans = 1;   // transforms of a pass
   int ntrans0 = 1;  // as it was created (gbn_plan_reserve raises ntrans)
   int spread_only = 0;
+  std::mutex calls;  // one call at a time: gbn_plan_reserve replaces arrays that others launch with
   int device = 0;
   int nsm = 152;
   double eps = 1e-6, sigma = 2.0, beta = 0.0;
@@ -644,6 +646,7 @@ template <typename F>
 int guarded(gbn_plan p, F&& f) {
   try {
     if (!p) fail(GBN_ERR_ARG, "null plan");
+    std::lock_guard<std::mutex> one(p->calls);
     DeviceGuard dg(p->device);
     f();
     return GBN_OK;
@@ -1469,7 +1472,9 @@ int gbn_toep_create(gbn_plan p, int64_t M, const float* k0, const float* k1, con
     // circulant grid and the kernel spectrum
     t = new gbn_toep_s();
     t->device = p->device;
-    chk(gbn_plan_create(g.dim, n1, 2.0, p->eps, p->ntrans, 0, p->device, &t->inner));
+    // as many transforms as the plan was created for: passes raised for other calls
+    // would multiply the circulant grids
+    chk(gbn_plan_create(g.dim, n1, 2.0, p->eps, p->ntrans0, 0, p->device, &t->inner));
     gbn_plan in = t->inner;
     ck(launch_toep_place(in->g, psf, in->fine, st), "Toeplitz placement");
     in->exec_fft(1, in->fine, -1, st, 0);

@@ -113,19 +113,27 @@ class MRIGB300(_Base):
         self.dtype = np.float32
         self._set_samples(samples)
         G = fine_cells(self.shape, self.eps, self.upsampfac)
-        self._cap = max(1, min(int(fine_budget_bytes // (8 * G)), 64))  # transforms of a pass
-        self._ntrans = max(1, min(max(n_batchs * n_coils, n_trans), self._cap))
+        self._budget = int(fine_budget_bytes // (8 * G))  # fine grids of the plan
+        self._ntrans = max(1, min(max(n_batchs * n_coils, n_trans), self._budget, 64))
+        self._grids = self._ntrans  # held: a grown plan keeps its old ones until it ends
         self._plan = NufftPlan(self.shape, self.eps, self.upsampfac, self._ntrans, device=self.device.index)
         self._plan.setpts(self._samples_d)
         self.compute_density(density)
         self.compute_smaps(smaps)
 
     def _reserve(self, transforms):
-        """Passes of up to ``transforms``, within the fine-grid budget."""
-        n = min(int(transforms), self._cap)
-        if n > self._ntrans:
+        """Passes of up to ``transforms`` (at most 64) where the fine-grid budget has
+        room for their grids next to those the plan holds already, and the device
+        memory for them; else passes stay as they are."""
+        n = min(int(transforms), 64, self._budget - self._grids)
+        if n <= self._ntrans:
+            return
+        try:
             self._plan.reserve(n)
-            self._ntrans = n
+        except MemoryError:
+            return
+        self._ntrans = n
+        self._grids += n
 
     # ----------------------------------------------------------------- state
     def _set_samples(self, samples, unsafe=False):

@@ -54,3 +54,39 @@ def test_captured_data_consistency_outlives_a_reserve(gpu_pkg):
     out.zero_()
     graph.replay()
     assert (torch.linalg.norm(out - want) / torch.linalg.norm(want)).item() < 1e-5
+
+
+def test_corrected_operator_within_the_budget(gpu_pkg, monkeypatch):
+    """The off-resonance wrapper raises its operator's passes only within the
+    fine-grid budget, old and new grids counted; without device memory for them
+    passes stay; the Toeplitz embedding of the operator does not grow."""
+    rng = np.random.default_rng(3)
+    shape, C, L, M = (32, 24), 4, 9, 400
+    k = rng.uniform(-0.5, 0.5, (M, 2)).astype(np.float32)
+    tup = _cpx(M, L).cpu().numpy(), _cpx(L, *shape).cpu().numpy()
+    smaps = _cpx(C, *shape)
+
+    def make(grids):
+        G = 64 * 48
+        return gpu_pkg.MRIGB300(k, shape, n_coils=C, smaps=smaps, squeeze_dims=False,
+                                fine_budget_bytes=8 * G * grids)
+
+    plain = make(100)
+    for grids, want in ((100, 36), (30, 26), (7, 4)):
+        op = make(grids)
+        held = op.plan.device_bytes
+        off = gpu_pkg.MRIFourierCorrectedGB300(op, interpolator=tup)
+        assert op.plan.ntrans == want
+        assert op.plan.device_bytes - held <= 8 * 64 * 48 * (grids - 4)
+        off.compute_interpolator(tup, None, None, None)  # again: no more than the budget
+        assert op.plan.device_bytes - held <= 8 * 64 * 48 * (grids - 4)
+        assert op._toeplitz().inner_device_bytes() == plain._toeplitz().inner_device_bytes()
+    op = make(100)
+
+    def full(n):
+        raise MemoryError("no room")
+
+    monkeypatch.setattr(op.plan, "reserve", full)
+    off = gpu_pkg.MRIFourierCorrectedGB300(op, interpolator=tup)
+    assert op.plan.ntrans == 4
+    assert off.op(_cpx(1, 1, *shape)).shape == (1, C, M)
