@@ -95,6 +95,16 @@ int gbn_plan_tune(gbn_plan plan, const int* bins, int interp_method, int maxsub_
 int gbn_plan_reserve(gbn_plan plan, int ntrans);
 
 /*
+ * The tensor-core kernels give up a wait after about a second; what they computed is
+ * then not valid.  The next call on the plan reports that as GBN_ERR_CUDA, once.  A
+ * caller that has synchronised and is about to use results (those of a replayed
+ * graph too, or of the last call) asks for it here.
+ */
+int gbn_plan_check(gbn_plan plan);
+/* The word of host memory that those kernels set (null: the plan uses none). */
+int gbn_plan_error_word(gbn_plan plan, int** word);
+
+/*
  * Set the non-uniform points: M samples, one float32 device array per image
  * axis (k2 ignored in 2D).  Bin-sorts the points on the device.  Replaces
  * Plan.setpts (finufft.py:55-62, cufinufft.py:94-113).

@@ -44,6 +44,8 @@ SIGNATURES = {
     "gbn_plan_device_bytes": (_c_int, [_vp, ctypes.POINTER(_c_i64)]),
     "gbn_plan_tune": (_c_int, [_vp, ctypes.POINTER(_c_int), _c_int, _c_int]),
     "gbn_plan_reserve": (_c_int, [_vp, _c_int]),
+    "gbn_plan_check": (_c_int, [_vp]),
+    "gbn_plan_error_word": (_c_int, [_vp, ctypes.POINTER(ctypes.POINTER(_c_int))]),
     "gbn_setpts": (_c_int, [_vp, _c_i64, _vp, _vp, _vp, _vp]),
     "gbn_op": (_c_int, [_vp, _vp, _vp, _vp, _c_int, _c_int, _c_flt, _c_int, _vp]),
     "gbn_adj": (_c_int, [_vp, _vp, _vp, _vp, _vp, _c_int, _c_int, _c_flt, _c_int, _vp]),

@@ -210,4 +210,11 @@ class BatchedNufft:
     def replay(self):
         if self.graph is None:
             self.capture()
+        self.check()  # a replayed graph does not look itself
         self.graph.replay()
+
+    def check(self):
+        """Raise if a kernel of a finished step gave up waiting (``NufftPlan.check``);
+        call it after synchronising, before results of a replay are used."""
+        for plan in self.plans:
+            plan.check()

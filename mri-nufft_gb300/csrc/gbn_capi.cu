@@ -147,6 +147,55 @@ std::vector<float> deconv_factors(int N, int64_t nf, int w, double beta) {
 
 }  // namespace
 
+namespace {
+
+// Words of page-locked host memory that tensor-core kernels set when a wait runs
+// out, one for each plan that uses such kernels.  The first 1024 living plans share
+// one page, kept for the process; each of any others has an allocation of its own.
+class ErrorWords {
+ public:
+  int* take() {
+    std::lock_guard<std::mutex> lk(mu_);
+    if (!page_) {
+      page_ = alloc(kWords);
+      for (int i = kWords; i-- > 0;) free_.push_back(page_ + i);
+    }
+    if (free_.empty()) return alloc(1);
+    int* const w = free_.back();
+    free_.pop_back();
+    *w = 0;
+    return w;
+  }
+  // no kernel of the plan is in flight any more
+  void give(int* w) {
+    if (!w) return;
+    std::lock_guard<std::mutex> lk(mu_);
+    if (w >= page_ && w < page_ + kWords) free_.push_back(w);  // capacity: never reallocates
+    else cudaFreeHost(w);
+  }
+
+ private:
+  static constexpr int kWords = 1024;
+  std::mutex mu_;
+  int* page_ = nullptr;
+  std::vector<int*> free_;
+  int* alloc(int n) {
+    free_.reserve(kWords);
+    int* p = nullptr;
+    ck(cudaHostAlloc(reinterpret_cast<void**>(&p), n * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped),
+       "error words");
+    std::memset(p, 0, n * sizeof(int));
+    return p;
+  }
+};
+
+ErrorWords& error_words() {
+  static ErrorWords* const w = new ErrorWords;  // outlives every plan
+  return *w;
+}
+
+}  // namespace
+
 void gbn::set_last_error(const char* msg) { g_err = msg; }
 
 struct gbn_plan_s {
@@ -165,6 +214,7 @@ struct gbn_plan_s {
   float2* kbuf = nullptr;  // ntrans x M residual scratch for dc
   std::vector<void*> retired;  // arrays replaced while work or captured graphs may use them
   unsigned* fmax = nullptr;  // ntrans: largest fine cell of each transform (2D tensor-core interp)
+  int* err = nullptr;      // the plan's error word (tensor-core kernels)
   int64_t kbuf_cap = 0;
   int64_t kbuf_M = 0;      // samples it was last used for
 
@@ -244,6 +294,7 @@ struct gbn_plan_s {
     free_points();
     free_bins();
     dev_free(sb.d_total);
+    error_words().give(err);  // after the frees, which wait for the device
   }
 
   void free_bins() {
@@ -437,18 +488,12 @@ void gbn_plan_s::exec_fft(int batch, float2* data, int isign, cudaStream_t st, i
 
 namespace {
 
-// A word of page-locked host memory that a tensor-core kernel sets when a wait
-// runs out; looked at by every later call.  Allocated once, by the first plan
-// that uses such a kernel.
-int* tc_error_flag() {
-  static int* const flag = [] {
-    int* f = nullptr;
-    ck(cudaHostAlloc(reinterpret_cast<void**>(&f), sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped),
-       "error flag");
-    *f = 0;
-    return f;
-  }();
-  return flag;
+// Reports, once, a wait that ran out in an earlier call on this plan.
+void check_waits(gbn_plan p) {
+  volatile int* const w = p->err;
+  if (!w || !*w) return;
+  *w = 0;
+  fail(GBN_ERR_CUDA, "a tensor-core kernel of this plan gave up waiting: results since the last check are not valid");
 }
 
 // what a plan with tensor-core tables needs beyond them
@@ -456,14 +501,13 @@ void setup_tc(gbn_plan p) {
   if (!p->tc) return;
   ck(tc_spread_prepare(), "spread kernel attributes");
   ck(tc_interp_prepare(), "interp kernel attributes");
-  tc_error_flag();
+  if (!p->err) p->err = error_words().take();
   if (!p->fmax && p->fft2d) p->fmax = dev_alloc<unsigned>(p->ntrans, p->bytes, "fine-grid maxima");
 }
 
 void require_points(gbn_plan p) {
   if (!p) fail(GBN_ERR_ARG, "null plan");
-  if (p->tc && *reinterpret_cast<volatile int*>(tc_error_flag()))
-    fail(GBN_ERR_CUDA, "a tensor-core kernel gave up waiting; its results are not valid");
+  check_waits(p);
   if (p->M < 0) fail(GBN_ERR_STATE, "gbn_setpts has not been called on this plan");
 }
 
@@ -489,7 +533,7 @@ void run_interp(gbn_plan p, const InterpArgs& a, cudaStream_t st) {
     InterpArgs t = a;
     t.s = p->sorted_spread();
     t.fmax = p->fmax;
-    ck(launch_interp_tc(t, tc_error_flag(), st), "interp kernel");
+    ck(launch_interp_tc(t, p->err, st), "interp kernel");
     p->launches++;
     return;
   }
@@ -503,7 +547,7 @@ void run_spread(gbn_plan p, const SpreadArgs& a, cudaStream_t st) {
   // warp-cooperative one (any sort order) for a single transform
   const bool stream = p->stream_spread && (a.g.dim == 3 || a.ntr >= 2);
   if (stream && p->tc) {
-    ck(launch_spread_tc(a, tc_error_flag(), st), "spread kernel");
+    ck(launch_spread_tc(a, p->err, st), "spread kernel");
     p->launches++;
     return;
   }
@@ -868,6 +912,17 @@ int gbn_plan_device_bytes(gbn_plan p, int64_t* bytes) {
   }
   *bytes = p->bytes;
   return GBN_OK;
+}
+
+int gbn_plan_check(gbn_plan p) {
+  return guarded(p, [&] { check_waits(p); });
+}
+
+int gbn_plan_error_word(gbn_plan p, int** word) {
+  return guarded(p, [&] {
+    if (!word) fail(GBN_ERR_ARG, "null argument");
+    *word = p->err;
+  });
 }
 
 int gbn_setpts(gbn_plan p, int64_t M, const float* k0, const float* k1, const float* k2,
@@ -1483,6 +1538,7 @@ int gbn_toep_create(gbn_plan p, int64_t M, const float* k0, const float* k1, con
     in->bytes += kb;
     ck(launch_real_part(in->fine, t->K, in->g.G, 1.0f, st), "Toeplitz kernel");
     ck(cudaStreamSynchronize(st), "Toeplitz kernel sync");
+    check_waits(q);
   });
   {
     DeviceGuard dg(p ? p->device : 0);

@@ -332,20 +332,20 @@ class MRIFourierCorrectedGB300:
         """Forward operator with the off-resonance effect (off_resonance.py:233-282)."""
         like = _array.interface_of(data)
         x = _array.to_tensor(data, self._fourier_op.device, torch.complex64)
-        return _array.from_tensor(self._squeeze(self._op_device(x)), like)
+        return self._fourier_op.plan.to_caller(self._squeeze(self._op_device(x)), like)
 
     def adj_op(self, coeffs, *args):
         """Adjoint operator with the off-resonance effect (off_resonance.py:284-332)."""
         like = _array.interface_of(coeffs)
         y = _array.to_tensor(coeffs, self._fourier_op.device, torch.complex64)
-        return _array.from_tensor(self._squeeze(self._adj_device(y)), like)
+        return self._fourier_op.plan.to_caller(self._squeeze(self._adj_device(y)), like)
 
     def data_consistency(self, image_data, obs_data):
         like = _array.interface_of(image_data)
         op = self._fourier_op
         x = _array.to_tensor(image_data, op.device, torch.complex64)
         y = _array.to_tensor(obs_data, op.device, torch.complex64).reshape(op.n_batchs, op.n_coils, -1)
-        return _array.from_tensor(self._squeeze(self._adj_device(self._op_device(x) - y)), like)
+        return self._fourier_op.plan.to_caller(self._squeeze(self._adj_device(self._op_device(x) - y)), like)
 
     def get_lipschitz_cst(self, max_iter=10, **kwargs):
         """Power method on the corrected operator with one coil and no maps
@@ -371,6 +371,7 @@ class MRIFourierCorrectedGB300:
                     break
                 x_norm = x_new_norm
                 x = x_new
+            op.plan.check()
             return x_new_norm
         finally:
             op._smaps, op._n_coils, op._n_batchs = smaps, C, B

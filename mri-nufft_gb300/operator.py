@@ -395,7 +395,7 @@ class MRIGB300(_Base):
         B, C, M = self.n_batchs, self.n_coils, self.n_samples
         out = _array.pinned_empty((B, C, M), torch.complex64)
         if out is None:  # the host cannot lock that much memory: one call, pageable copy
-            return _array.from_tensor(self._op_device(self._img_tensor(data)), _array.Interface("numpy"))
+            return self._plan.to_caller(self._op_device(self._img_tensor(data)), _array.Interface("numpy"))
         x = self._img_tensor(data)
         dev_k = torch.empty((B, C, M), dtype=torch.complex64, device=self.device)
         main = torch.cuda.current_stream(self.device)
@@ -412,6 +412,7 @@ class MRIGB300(_Base):
                 with torch.cuda.stream(side):
                     out[b, c0:c1].copy_(dev_k[b, c0:c1], non_blocking=True)
         side.synchronize()
+        self._plan.check()
         return out.numpy()
 
     def _op(self, image, coeffs):
@@ -435,8 +436,9 @@ class MRIGB300(_Base):
                 return out_buf
             if isinstance(out_buf, np.ndarray):
                 np.copyto(out_buf, ret.reshape(out_buf.shape).cpu().numpy())
+                self._plan.check()
                 return out_buf
-        return _array.from_tensor(ret, like)
+        return self._plan.to_caller(ret, like)
 
     def data_consistency(self, image_data, obs_data):
         """Gradient of the data-consistency term A^H(Ax - y), fused per pass."""
@@ -446,7 +448,7 @@ class MRIGB300(_Base):
         out = torch.empty(self.img_full_shape, dtype=torch.complex64, device=self.device)
         B, C = self.n_batchs, self.n_coils
         self._plan.dc(x, y, self._density, self._smaps, out, B, C, self.inv_norm_factor)
-        return _array.from_tensor(self._safe_squeeze(out), like)
+        return self._plan.to_caller(self._safe_squeeze(out), like)
 
     def gram_op(self, data, toeplitz=True):
         """Gram operator A^H W A x (base.py:315-363).  ``toeplitz=True`` uses
@@ -627,6 +629,7 @@ def power_method(max_iter, operator: MRIGB300, x: torch.Tensor, toeplitz=False):
             x = x_new
         if i == max_iter - 1:
             warnings.warn("Lipschitz constant did not converge")
+        operator._plan.check()
         return x_new_norm
     finally:
         operator._smaps = smaps

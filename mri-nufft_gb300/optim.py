@@ -109,7 +109,7 @@ def cg(operator, kspace_data, damp=0.0, x0=None, x_init=None, max_iter=10, tol=1
                                         damp=damp, x0=x0))
         if operator.squeeze_dims:
             image = operator._safe_squeeze(image)
-        out = _array.from_tensor(image, like)
+        out = operator.plan.to_caller(image, like)
     finally:
         if old_density is not None:
             operator._density = old_density
@@ -284,7 +284,7 @@ def lsqr(operator, kspace_data, damp=0.0, atol=1e-6, btol=1e-6, conlim=1e8, max_
 def _finish(operator, x, like, results, old_density):
     if operator.squeeze_dims:
         x = operator._safe_squeeze(x)
-    out = _array.from_tensor(x, like)
+    out = operator.plan.to_caller(x, like)
     if results:
         return out, results
     return out

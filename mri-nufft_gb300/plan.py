@@ -14,7 +14,7 @@ import ctypes
 
 import torch
 
-from . import _lib
+from . import _array, _lib
 
 
 def _ptr(t):
@@ -99,6 +99,18 @@ class NufftPlan:
         """Raise the transforms of a pass to at least ``ntrans``."""
         _lib.check(self.lib.gbn_plan_reserve(self._h, int(ntrans)), "gbn_plan_reserve")
         self.ntrans = max(self.ntrans, int(ntrans))
+
+    def check(self):
+        """Raise if a kernel of an earlier, finished call gave up waiting, so that its
+        results are not valid (``gbn_plan_check``)."""
+        _lib.check(self.lib.gbn_plan_check(self._h), "gbn_plan_check")
+
+    def to_caller(self, t, like):
+        """``t`` in the caller's array type; results on the host are finished and checked."""
+        out = _array.from_tensor(t, like)
+        if like.kind == "numpy" or like.kind == "torch" and like.device.type == "cpu":
+            self.check()
+        return out
 
     def _reset_points(self):
         cols = self._coords

@@ -304,9 +304,15 @@ class _Solve:
                 self._ck(self.lib.gbn_cg_update(nimg, _ptr(gnew), _ptr(grad), _ptr(velocity),
                                                 _ptr(image), _ptr(st), _ptr(L), tol, sth), "cg update")
             yield
-        self.image = image
+        self._image = image
         self.event = torch.cuda.Event()
         self.event.record(self.stream)
+
+    @property
+    def image(self):
+        """The result, once ``event`` has passed; raises if a kernel gave up waiting."""
+        self.plan.check()
+        return self._image
 
     def step(self):
         """Issue the next unit; False once every unit is issued."""

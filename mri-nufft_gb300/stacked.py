@@ -215,7 +215,7 @@ class MRIStackedGB300(_Base):
         x = _array.to_tensor(image_data, self.device, torch.complex64)
         y = _array.to_tensor(obs_data, self.device, torch.complex64).reshape(self.n_batchs, self.n_coils, -1)
         r = self._op_device(x) - y
-        return _array.from_tensor(self._safe_squeeze(self._adj_device(r)), like)
+        return self.operator.plan.to_caller(self._safe_squeeze(self._adj_device(r)), like)
 
     def get_lipschitz_cst(self, max_iter=10):
         """The 2D operator's Lipschitz constant, as the reference (stacked.py:418-438)."""
@@ -228,5 +228,6 @@ class MRIStackedGB300(_Base):
                 return out_buf
             if isinstance(out_buf, np.ndarray):
                 np.copyto(out_buf, ret.reshape(out_buf.shape).cpu().numpy())
+                self.operator.plan.check()
                 return out_buf
-        return _array.from_tensor(ret, like)
+        return self.operator.plan.to_caller(ret, like)
