@@ -145,23 +145,9 @@ class MRIGB300(_Base):
             raise ValueError(f"samples must have {len(self.shape)} columns")
         t = _array.to_tensor(s, self.device, torch.float32).reshape(-1, len(self.shape))
         self._samples_d = t
-        self._samples = None
-
-    # The host copy of the samples is made when it is asked for: the copy and the
-    # Fortran order of 2.1 M 3D samples took 14 ms of every operator's creation.
-    @property
-    def _samples(self):
-        if self._samples_host is None:
-            # from the plan's own columns: the caller may have changed its array
-            out = np.empty((self.n_samples, len(self.shape)), dtype=np.float32, order="F")
-            for d, col in enumerate(self._plan._coords[:len(self.shape)]):
-                out[:, d] = col.cpu().numpy()
-            self._samples_host = out
-        return self._samples_host
-
-    @_samples.setter
-    def _samples(self, value):
-        self._samples_host = value
+        # the host copy is made now, Fortran-ordered: columns side by side on the device
+        # are that order (2.1 M 3D samples 0.19 ms; by rows, turned on the host, 5.5)
+        self._samples = t.t().contiguous().cpu().numpy().T
 
     @property
     def samples(self):
