@@ -592,7 +592,7 @@ void run_fft_crop(gbn_plan p, const CropArgs& a, int isign, cudaStream_t st) {
     Span span(p, GBN_STAGE_FFT, st);
     ck(launch_fft2d_adj(a, const_cast<float2*>(a.fine), p->twiddles(), isign, st),
        "fused transform + crop");
-    p->launches += 2;
+    p->launches += a.smaps && a.ntr > 1 ? 3 : 2;
     return;
   }
   if (p->fft3d) {
@@ -1477,7 +1477,7 @@ void toep_apply(gbn_toep t, const void* img, const void* smaps, void* out, int B
     if (p->fft2d && g.nf[0] == 512) {
       Span span(p, GBN_STAGE_FFT, st);
       ck(launch_fft2d_gram(pa, ca, t->K, p->twiddles(), st), "fused Toeplitz Gram");
-      p->launches += 3;
+      p->launches += ca.smaps && T > 1 ? 4 : 3;
       return;
     }
     run_pad_fft(p, pa, -1, st);
