@@ -243,6 +243,7 @@ struct gbn_plan_s {
   int* ssub = nullptr;     // spread chunk table, 3 x sscap
   int64_t sscap = 0;
   int nsub_s = 0;
+  int nzb = 0;             // 3D with `tc`: occupied (column, block of 8 z cells) pairs
   int maxsub_s = 0;
 
   std::map<int, cufftHandle> ffts;
@@ -540,13 +541,52 @@ void run_interp(gbn_plan p, const InterpArgs& a, cudaStream_t st) {
   ck(a.g.dim == 2 ? launch_interp2d(a, st) : launch_interp3d(a, st), "interp kernel");
   p->launches++;
 }
+// Whether a pass of ntr transforms of a plan with tensor-core tables spreads on the
+// tensor cores.  Their kernels pay for a whole tile or z block whatever its samples, the
+// FP32 ones for each sample and transform.
+//
+// 3D, against the quadrant kernel on the same columns, by the samples a of an occupied
+// block of 8 z cells (256^3 cells, us, tensor cores / FP32): uniform samples, 4
+// transforms a = 1.0 96 / 73, 1.4 456 / 530; 3 transforms 1.4 429 / 389, 3.1 659 / 774;
+// 2 transforms 3.1 624 / 525, 11.8 788 / 855, radial 11.4 291 / 279, 22 610 / 655; one
+// 11.8 631 / 528, radial 22 506 / 435, 44 65 / 74.  Narrower kernels (4 transforms):
+// w = 5 a = 1.9 319 / 320, w = 4 2.3 269 / 220.  Below 32 768 samples the columns are too
+// few to fill the GPU and the FP32 kernel is the shorter chain: radial 16 384, 4
+// transforms, a = 8 62 / 52.
+//
+// 2D, against per-sample atomics, whose cost is estimated with the rates of 128^2 to
+// 2000^2 cells: 512^2 cells, 16 384 samples on 2700 tiles, 2 / 8 / 32 transforms 35 / 35
+// / 70 on the tensor cores, 10 / 21 / 59 by sample; 65 536 samples, 2 / 4 / 8 transforms
+// 37 / 39 / 40 and 19 / 29 / 50.
+bool tc_spread_pays(gbn_plan p, int ntr) {
+  const Geom& g = p->g;
+  if (g.method_spread == 6) return true;
+  const double M = (double)p->M;
+  if (g.dim == 3) {
+    const double narrow = std::pow(7.0 / g.w, 1.5);
+    const double need = ntr == 1 ? 32.0 : ntr == 2 ? 12.0 : ntr == 3 ? 3.0 : (ntr < 7 && ntr > 4 ? 2.0 : 1.3) * narrow;
+    return M >= 32768 && M >= need * p->nzb;
+  }
+  if (ntr < 2) return false;
+  // tiles take 12 ns each, 24 in groups of 32 transforms; a sample and transform 0.1 ns
+  // (w = 7, warp-cooperative) or 0.15 for 25 cells, in a chain of 0.35 or 3.5 us a transform
+  const double tile = ntr > 16 ? 0.0244 * ((ntr + 31) / 32) : 0.0122;
+  const double tc = 5.0 + tile * p->nsub_s + 5e-5 * M;
+  const double cells = g.w * g.w / 25.0;
+  const double chain = g.w == 7 ? 6.0 + 0.35 * ntr : 8.0 + 3.5 * ntr * cells;
+  const double work = g.w == 7 ? 1e-4 * M * ntr : 1.5e-4 * cells * M * ntr;
+  return tc < (g.w == 7 ? chain + work : std::fmax(chain, 8.0 + work));
+}
+
 void run_spread(gbn_plan p, const SpreadArgs& a, cudaStream_t st) {
   if (a.s.nsub == 0) return;
   Span span(p, GBN_STAGE_SPREAD, st);
   // 2D: the streaming spreader for several transforms per call, the
-  // warp-cooperative one (any sort order) for a single transform
-  const bool stream = p->stream_spread && (a.g.dim == 3 || a.ntr >= 2);
-  if (stream && p->tc) {
+  // warp-cooperative one (any sort order) for a single transform and for samples that
+  // do not pay a tile
+  const bool on_tc = p->tc && tc_spread_pays(p, a.ntr);
+  const bool stream = p->stream_spread && (a.g.dim == 3 || (a.ntr >= 2 && (on_tc || !p->tc)));
+  if (on_tc) {
     ck(launch_spread_tc(a, p->err, st), "spread kernel");
     p->launches++;
     return;
@@ -867,7 +907,7 @@ int gbn_plan_create(int dim, const int64_t* n_modes, double upsampfac, double ep
     p->fine = dev_alloc<float2>((size_t)ntrans * g.G, p->bytes, "fine grid");
     p->setup_bins();
     setup_tc(p);
-    p->sb.d_total = dev_alloc<int>(2, p->bytes, "scan");
+    p->sb.d_total = dev_alloc<int>(3, p->bytes, "scan");
     *out = p;
     return GBN_OK;
   } catch (const Fail& e) {
@@ -984,7 +1024,7 @@ int gbn_setpts(gbn_plan p, int64_t M, const float* k0, const float* k1, const fl
     const float* k[3] = {k0, k1, k2};
     p->maxsub = maxsub_i;
     p->maxsub_s = maxsub_s;
-    int totals[2] = {0, 0};
+    int totals[3] = {0, 0, 0};
     if (p->stream_spread) {
       const Geom& g = p->g;
       const int last = g.dim - 1;
@@ -1005,6 +1045,8 @@ int gbn_setpts(gbn_plan p, int64_t M, const float* k0, const float* k1, const fl
       ck(build_group_table(ns, ns / p->ncol, p->sgrp_k, g.nkey[last], maxsub_s, p->sb, gc,
                            p->sb.d_total + 1, st),
          "spread chunks");
+      if (p->tc && g.dim == 3)
+        ck(count_zblocks(g, p->ncol, M, p->sb, p->sb.d_total + 2, st), "spread blocks");
     } else {
       ck(sort_points(p->g, M, k, maxsub, p->sb, st, true), "sort");
     }
@@ -1015,6 +1057,7 @@ int gbn_setpts(gbn_plan p, int64_t M, const float* k0, const float* k1, const fl
     if (total > p->subcap || (p->stream_spread && totals[1] > p->sscap))
       fail(GBN_ERR_CUDA, "subproblem table overflow");
     p->nsub_s = p->stream_spread ? totals[1] : 0;
+    p->nzb = p->tc && p->g.dim == 3 ? totals[2] : 0;
     p->nsub = total;
     p->M = M;
   });

@@ -1325,7 +1325,11 @@ __device__ __forceinline__ void stream_flush_mask2(unsigned mask, int zb, float2
 // a sample occupies about 3 of the 4 warps.  Quadrant cross-sections overlap
 // by w rows, which the float2 flush atomics absorb.  The z window, rotated
 // weights and flush rules are those of the column kernel.
+//
+// Columns whose whole cross-section is at most 11 x 11 rows (those of the
+// tensor-core spreader) are one CTA instead of four.
 // ---------------------------------------------------------------------------
+inline __host__ __device__ bool quad_whole(const Geom& g) { return g.pd[0] <= 11 && g.pd[1] <= 11; }
 constexpr int kQuadThreads = 128;
 constexpr int kQuadRound = 256;  // samples staged at a time
 
@@ -1353,19 +1357,20 @@ spread_quad3d_kernel(SpreadArgs a) {
   const Geom& g = a.g;
   // the four quadrants of a chunk are consecutive blocks, so that they run
   // together and their overlapping rows meet in L2
-  const int sub = blockIdx.x >> 2;
+  const bool whole = quad_whole(g);
+  const int sub = whole ? blockIdx.x : blockIdx.x >> 2;
   const int col = a.s.sub_bin[sub];
   const int p0 = a.s.sub_start[sub];
   const int cnt = imin(a.s.sub_count[sub], kStreamBatch);
   const int w = W > 0 ? W : g.w;
-  const int qx = (blockIdx.x >> 1) & 1, qy = blockIdx.x & 1;
+  const int qx = whole ? 0 : (blockIdx.x >> 1) & 1, qy = whole ? 0 : blockIdx.x & 1;
   const int b0 = (col / g.nb[1]) * g.bs[0] - g.koff;  // column origin (footprint frame)
   const int b1 = (col % g.nb[1]) * g.bs[1] - g.koff;
   const int o0 = b0 + 4 * qx, o1 = b1 + 4 * qy;   // quadrant origin
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int pdq = 4 + w;
+  const int nrx = whole ? g.pd[0] : 4 + w, pdq = whole ? g.pd[1] : 4 + w;  // rows along x, y
   const int i0 = threadIdx.x / pdq, i1 = threadIdx.x - i0 * pdq;
-  const bool own = (int)threadIdx.x < pdq * pdq;
+  const bool own = (int)threadIdx.x < nrx * pdq;
   const int nf2 = g.nf[2];
   const int G = (int)g.G;
   const int rowbase = own ? (wrap_idx(o0 + i0, g.nf[0]) * g.nf[1] + wrap_idx(o1 + i1, g.nf[1])) * nf2 : 0;
@@ -1378,7 +1383,7 @@ spread_quad3d_kernel(SpreadArgs a) {
     if (t < cnt) {
       const int a0 = (int)ceilf(a.s.u[0][p0 + t] - g.halfw) - b0;  // 0 .. 8
       const int a1 = (int)ceilf(a.s.u[1][p0 + t] - g.halfw) - b1;
-      mine = (a0 >= 4) == (qx == 1) && (a1 >= 4) == (qy == 1);
+      mine = whole || ((a0 >= 4) == (qx == 1) && (a1 >= 4) == (qy == 1));
     }
     const unsigned bal = __ballot_sync(0xffffffffu, mine);
     if (lane == 0) s_wsum[warp] = __popc(bal);
@@ -1412,7 +1417,7 @@ spread_quad3d_kernel(SpreadArgs a) {
       unsigned wm = 0;
 #pragma unroll
       for (int q = 0; q < kQuadThreads / 32; ++q)
-        if (a0 <= imin((32 * q + 31) / pdq, pdq - 1) && a0 + w - 1 >= (32 * q) / pdq) wm |= 1u << q;
+        if (a0 <= imin((32 * q + 31) / pdq, nrx - 1) && a0 + w - 1 >= (32 * q) / pdq) wm |= 1u << q;
       s_hd[t] = (unsigned)(zs + 8) | ((unsigned)a0 << 16) | ((unsigned)a1 << 20) | (wm << 24);
     }
   };
@@ -2118,7 +2123,7 @@ cudaError_t launch_spread_quad_t(const SpreadArgs& a, cudaStream_t st) {
   auto k = spread_quad3d_kernel<W, CG, MINB, PACKED>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  k<<<(unsigned)(4 * (int64_t)a.s.nsub), kQuadThreads, smem, st>>>(a);
+  k<<<(unsigned)((quad_whole(a.g) ? 1 : 4) * (int64_t)a.s.nsub), kQuadThreads, smem, st>>>(a);
   return cudaGetLastError();
 }
 
@@ -2128,7 +2133,7 @@ inline cudaError_t dispatch_spread_stream3d(const SpreadArgs& a, cudaStream_t st
   if (a.g.spread_cg == 1 || a.g.spread_cg == 2 || a.g.spread_cg == 4) cg = imin(cg, a.g.spread_cg);
   // 8 x 8 bins: quadrant CTAs (measured 7 % faster than whole columns on the
   // 3D kooshball); GBN_SPREAD=stream keeps the column kernel
-  if ((a.g.method_spread == 0 || a.g.method_spread == 5) && a.g.bs[0] == 8 && a.g.bs[1] == 8) {
+  if (a.g.method_spread != 3 && (quad_whole(a.g) || (a.g.bs[0] == 8 && a.g.bs[1] == 8))) {
     if (a.g.w == 7) {
       // 4 coils per pass at 3 CTAs per SM (170 registers, no spills;
       // measured 7.08 against 7.63 ms at 4 CTAs per SM, whose 128-register

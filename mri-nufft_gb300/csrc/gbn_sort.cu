@@ -58,6 +58,24 @@ __global__ void scatter_kernel(Geom g, int64_t M, const float* __restrict__ k0,
   }
 }
 
+// Occupied (column, z block) pairs of a 3D column sort: the z block of a sample is
+// (first cell + 8) >> 3, as in the tensor-core spreader.  nl keys a column.
+__global__ void zblock_kernel(int ncol, int nl, int koff, int nblk, int nkeys, int M,
+                              const int* __restrict__ bin_start, int* __restrict__ n_out) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  bool on = false;
+  if (i < (int64_t)ncol * nblk) {
+    const int col = (int)(i / nblk), blk = (int)(i - (int64_t)col * nblk);
+    const int k0 = 8 * blk - 8 + koff < 0 ? 0 : 8 * blk - 8 + koff, k1 = imin(8 * blk + koff, nl);
+    if (k0 < k1) {
+      const int b0 = col * nl + k0, b1 = col * nl + k1;
+      on = bin_start[b0] < (b1 < nkeys ? bin_start[b1] : M);
+    }
+  }
+  const int n = __popc(__ballot_sync(0xffffffffu, on));
+  if ((threadIdx.x & 31) == 0 && n) atomicAdd(n_out, n);
+}
+
 __global__ void nsub_kernel(int nbins, const int* __restrict__ bin_count, int maxsub,
                             int* __restrict__ nsub) {
   int b = blockIdx.x * blockDim.x + threadIdx.x;
@@ -209,6 +227,16 @@ cudaError_t build_group_table(int ngroups, int ngz, int K, int nl, int maxsub,
   if (e != cudaSuccess) return e;
   fill_sub_kernel<<<bb, 256, 0, st>>>(ngroups, gb.grp_count, gb.grp_start, gb.grp_off, maxsub,
                                       gb.sub_bin, gb.sub_start, gb.sub_count);
+  return cudaGetLastError();
+}
+
+cudaError_t count_zblocks(const Geom& g, int ncol, int64_t M, const SortBuffers& sb, int* d_out, cudaStream_t st) {
+  cudaError_t e = cudaMemsetAsync(d_out, 0, sizeof(int), st);
+  if (e != cudaSuccess) return e;
+  const int nl = g.nkey[2], nblk = ((g.nf[2] + 7) >> 3) + 1;
+  const int64_t n = (int64_t)ncol * nblk;
+  zblock_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(ncol, nl, g.koff, nblk, ncol * nl, (int)M, sb.bin_start,
+                                                             d_out);
   return cudaGetLastError();
 }
 

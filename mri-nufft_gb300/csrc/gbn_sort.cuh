@@ -44,6 +44,8 @@ cudaError_t build_group_table(int ngroups, int ngz, int K, int nl, int maxsub,
                               cudaStream_t st);
 cudaError_t exclusive_scan(const int* in, int* out, int n, int* scratch, int* total,
                            cudaStream_t st);
+// The occupied (column, block of 8 z cells) pairs of a finished 3D column sort.
+cudaError_t count_zblocks(const Geom& g, int ncol, int64_t M, const SortBuffers& sb, int* d_out, cudaStream_t st);
 // Sorts M points with coordinates k[d] (radians, device float32) by the bins
 // of g.  With `subproblems`, also cuts every bin into subproblems of at most
 // maxsub samples; on return (stream-ordered) sb.d_total holds their number.
