@@ -1039,10 +1039,10 @@ int gbn_setpts(gbn_plan p, int64_t M, const float* k0, const float* k1, const fl
       const int ns = p->sgrp_n;
       GroupBuffers gc{q, q + ns, q + 2 * (size_t)ns, q + 3 * (size_t)ns,
                       p->ssub, p->ssub + p->sscap, p->ssub + 2 * p->sscap};
-      ck(build_group_table(p->ngrp, g.nb[last], g.bs[last], g.nkey[last], maxsub_i, p->sb, gi,
+      ck(build_group_table(p->ngrp, g.nb[last], g.bs[last], g.nkey[last], M, maxsub_i, p->sb, gi,
                            p->sb.d_total, st),
          "interp groups");
-      ck(build_group_table(ns, ns / p->ncol, p->sgrp_k, g.nkey[last], maxsub_s, p->sb, gc,
+      ck(build_group_table(ns, ns / p->ncol, p->sgrp_k, g.nkey[last], M, maxsub_s, p->sb, gc,
                            p->sb.d_total + 1, st),
          "spread chunks");
       if (p->tc && g.dim == 3)

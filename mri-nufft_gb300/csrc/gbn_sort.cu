@@ -101,8 +101,10 @@ __global__ void fill_sub_kernel(int nbins, const int* __restrict__ bin_count,
 
 // Groups of K consecutive bins along the last axis (bins of one column are
 // contiguous in the sorted order): group gi = column * ngz + gz covers the
-// bins of layers [gz*K, min(nl, gz*K + K)) of its column.
-__global__ void group_kernel(int ngroups, int ngz, int K, int nl, const int* __restrict__ bin_count,
+// bins of layers [gz*K, min(nl, gz*K + K)) of its column.  Its size is the
+// difference of two bin starts: a sum over the counts of a column is one thread's
+// chain of nl reads (gbn_setpts, 400^3 cells, 2 M samples: 314 -> 300 us).
+__global__ void group_kernel(int ngroups, int ngz, int K, int nl, int nbins, int M,
                              const int* __restrict__ bin_start, int* __restrict__ grp_count,
                              int* __restrict__ grp_start) {
   int gi = blockIdx.x * blockDim.x + threadIdx.x;
@@ -111,10 +113,9 @@ __global__ void group_kernel(int ngroups, int ngz, int K, int nl, const int* __r
   const int l0 = gz * K;
   const int l1 = imin(nl, l0 + K);
   const int64_t b = (int64_t)col * nl;
-  int c = 0;
-  for (int l = l0; l < l1; ++l) c += bin_count[b + l];
-  grp_count[gi] = c;
-  grp_start[gi] = bin_start[b + l0];
+  const int start = bin_start[b + l0];
+  grp_count[gi] = (b + l1 < nbins ? bin_start[b + l1] : M) - start;
+  grp_start[gi] = start;
 }
 
 // ---------------------------------------------------------------------------
@@ -216,11 +217,11 @@ cudaError_t exclusive_scan(const int* in, int* out, int n, int* scratch, int* to
   return cudaGetLastError();
 }
 
-cudaError_t build_group_table(int ngroups, int ngz, int K, int nl, int maxsub,
+cudaError_t build_group_table(int ngroups, int ngz, int K, int nl, int64_t M, int maxsub,
                               const SortBuffers& sb, const GroupBuffers& gb, int* d_total,
                               cudaStream_t st) {
   int bb = (ngroups + 255) / 256;
-  group_kernel<<<bb, 256, 0, st>>>(ngroups, ngz, K, nl, sb.bin_count, sb.bin_start, gb.grp_count,
+  group_kernel<<<bb, 256, 0, st>>>(ngroups, ngz, K, nl, ngroups / ngz * nl, (int)M, sb.bin_start, gb.grp_count,
                                    gb.grp_start);
   nsub_kernel<<<bb, 256, 0, st>>>(ngroups, gb.grp_count, maxsub, gb.nsub_grp);
   cudaError_t e = exclusive_scan(gb.nsub_grp, gb.grp_off, ngroups, sb.scan_scratch, d_total, st);

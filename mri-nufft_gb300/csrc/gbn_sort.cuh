@@ -39,7 +39,7 @@ constexpr int kMaxBins = 2147483647 - 8192;
 size_t scan_scratch_ints(int n);
 // Builds gb's subproblem table (chunks of <= maxsub samples per group) from a
 // finished sort; d_total receives the number of subproblems.
-cudaError_t build_group_table(int ngroups, int ngz, int K, int nl, int maxsub,
+cudaError_t build_group_table(int ngroups, int ngz, int K, int nl, int64_t M, int maxsub,
                               const SortBuffers& sb, const GroupBuffers& gb, int* d_total,
                               cudaStream_t st);
 cudaError_t exclusive_scan(const int* in, int* out, int n, int* scratch, int* total,
