@@ -2239,12 +2239,19 @@ inline cudaError_t launch_interp_twc(const InterpArgs& a, cudaStream_t st) {
 template <int DIM>
 cudaError_t dispatch_interp(const InterpArgs& a, cudaStream_t st) {
   if constexpr (DIM == 2) {
-    // 4 tiles at a time, whose cells serve all samples on them: 8 / 16 / 24 radial
-    // transforms on 512^2 cells (0.5 samples a cell) 43 / 72 / 104 -> 37 / 58 / 80 us
-    // against the warp-cooperative kernel, 2 25 -> 21; 768^2 (0.22) 41 / 71 / 111 ->
-    // 41 / 64 / 87, 3 27 -> 29; 0.1 samples a cell, 16 transforms 25 -> 32
+    // 4 tiles at a time, whose 480 cells serve up to 64 samples: against the
+    // warp-cooperative kernel where the subproblems are full enough and enough to fill
+    // the GPU (each CTA takes the transforms in turn).  us, tiles / gather: radial, 512^2
+    // cells, 52 samples a subproblem, 2535 of them, 2 / 8 / 16 transforms 21 / 37 / 58 and
+    // 25 / 43 / 72; spiral, 768^2, 45, 2939 of them, 16 64 / 71; uniform samples, 512^2, 42,
+    // 4 / 16 27 / 65 and 24 / 60; 256^2, 53, 622 of them, 4 / 8 / 16 15 / 21 / 30 and
+    // 14 / 19 / 31; 128^2, 56, 291 of them, 4 / 64 12 / 62 and 10 / 49.  1490 subproblems
+    // (400^2, 54), a second round of CTAs that is mostly empty: 2 / 4 / 8 15 / 25 / 36 and
+    // 18 / 22 / 33.
+    const int64_t ns = a.s.nsub;
+    const bool few = a.s.M >= 50 * ns && ns >= 760 && (a.ntr == 2 || ns <= 1216 || ns >= 2128);
     if (a.g.tile2 && a.g.method_interp == 0 && a.ntr > 1 &&
-        (a.ntr > 8 ? 6 : 3) * a.s.M >= a.g.G)
+        (a.ntr > 8 ? a.s.M >= 44 * ns && ns >= 456 : few))
       return a.ntr > 2 ? dispatch_interp_w<2, 4>(a, st) : dispatch_interp_w<2, 2>(a, st);
   }
   // the rest of 2D at w = 7 takes the warp-cooperative direct kernel, 3D tiles;
