@@ -19,7 +19,9 @@
 // Nz / R terms per plane after one radix-R step (R = 4, 2 or 1, the largest that
 // divides Nz), and the work stack is never written: 1.1 GB a direction instead of
 // 3.2 GB for 256 x 256 x 64 and 16 coils, op + adj around the 2D transforms 3.2 ->
-// 1.0 ms (floor at the copy bandwidth 0.33; the forward sum is FP32-bound).
+// 1.0 ms (floor at the copy bandwidth 0.33; the forward sum is FP32-bound).  Their work
+// grows with planes squared, so long odd axes and small stacks keep the three passes
+// (fwd_in_one, adj_in_one).
 #include <cufft.h>
 
 #include <cmath>
@@ -460,6 +462,36 @@ int exec_z(cufftHandle h, float2* P, int dir, cudaStream_t st) {
   return GBN_OK;
 }
 
+// Whether the forward z transform runs as one kernel: a warp sums n4 terms for 8
+// planes at a time, 64 a round.  256 x 256, 8 coils (us, one kernel / three passes): 64
+// planes 165 / 502, 90 580 / 814, 55 (radix 1) 328 / 471, 65 507 / 545, 75 693 / 635; 32 x
+// 32, one coil: 7 / 13, 15 / 13, 9 / 13, 15 / 12, 17 / 13.
+bool fwd_in_one(const gbn_stack_s* s, int C) {
+  return s->radix && s->dft.n4 * ((s->dft.npad + 63) / 64) <= (s->g.nxy * C >= 4096 ? 100 : 80);
+}
+
+// The same for the adjoint, whose CTAs walk over the coils with maps.  Estimates in us
+// with rates measured on 32^2 to 256^2 x 9 to 126 planes and 1, 8 coils: the sum takes
+// 0.32 us a million terms, at least 8 ns a CTA and coil, or its chain where few columns
+// leave the GPU idle (14 ns a term of a warp, for every coil with maps); the three passes
+// 14.5 ps a cell while the stack stays in L2, up to 2.3 times that beyond.  128 x 128, 8
+// coils: 64 planes 98 / 127, 120 264 / 298, 45 (radix 1) 139 / 99, 75 332 / 163; 256 x
+// 256: 9 planes 121 / 76, 64 351 / 902; 32 x 32 with maps: 64 planes 35 / 21, 75 101 / 25.
+bool adj_in_one(const gbn_stack_s* s, int C, bool maps) {
+  if (!s->radix) return false;
+  const StackGeom& g = s->g;
+  const StackDft& d = s->dft;
+  const double cols = (double)g.nxy * C, cells = cols * g.nz, kept = cols * g.nzi;
+  const double chain = 0.0136 * ((d.n4 + 7) / 8) * d.npad;
+  const double lat = 5.5 + (maps ? C * (chain + 1.8) : chain);
+  const double sum = 7.0 + 0.32e-6 * cols * d.n4 * d.npad + 3.2e-6 * (cells + kept);
+  const double ctas = 7.0 + 0.0078 * cols / kDftCols;
+  const double one = maps ? std::fmax(1.13 * sum, 1.25 * ctas) : std::fmax(sum, ctas);
+  const double beyond = std::fmin(std::fmax((cells + kept - 20e6) / 45e6, 0.0), 1.3);
+  const double three = 13.0 + (1.0 + beyond) * (9e-6 * cells + 5.5e-6 * kept);
+  return std::fmax(lat, one) < (maps ? 0.88 : 1.0) * three;
+}
+
 // Tables of the one-kernel z transforms when the stack fits them: distinct planes
 // (a repeated one is written by an unspecified copy in the scatter) and tables
 // and columns within 96 KB of shared memory.
@@ -563,7 +595,7 @@ int gbn_stack_fwd(gbn_stack s, const void* img, const void* smaps, void* out, in
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const StackGeom& g = s->g;
   const float scale = (float)(1.0 / std::sqrt(2.0 * g.nz));
-  if (s->radix && C <= 65535) {
+  if (C <= 65535 && fwd_in_one(s, C)) {
     const float2 *x = static_cast<const float2*>(img), *m = static_cast<const float2*>(smaps);
     float2* const y = static_cast<float2*>(out);
     return ck_cuda(s->radix == 4   ? dft_fwd<4>(g, s->dft, x, m, y, C, scale, s->smem_fwd, st)
@@ -590,7 +622,7 @@ int gbn_stack_adj(gbn_stack s, const void* in, const void* smaps, void* img, int
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   const StackGeom& g = s->g;
   const float scale = (float)(1.0 / std::sqrt(2.0 * g.nz));
-  if (s->radix && C <= 65535) {
+  if (C <= 65535 && adj_in_one(s, C, smaps != nullptr)) {
     const float2 *y = static_cast<const float2*>(in), *m = static_cast<const float2*>(smaps);
     float2* const x = static_cast<float2*>(img);
     return ck_cuda(s->radix == 4   ? dft_adj<4>(g, s->dft, y, m, x, C, accumulate, scale, s->smem_adj, st)
