@@ -1955,13 +1955,14 @@ grad_kernel(GradArgs a, int conj_a) {
   bin_origin<DIM>(g, b, o);
   const int T = g.tile;
   const int w = W > 0 ? W : g.w;
-  const int WL = W > 0 ? W : w;
 
   __shared__ int s_rowoff[kMaxTileRows];
   const int* rowoff = tile_rows_init<DIM>(g, o, s_rowoff);
   __syncthreads();
   for (int c = 0; c < a.ntr; ++c) {
-    load_tiles<DIM>(tile, a.fine, g, o, c, 1, rowoff);
+    load_tile_async<DIM>(tile, a.fine + (int64_t)c * g.G, g, o, rowoff);
+    cp_async_commit();
+    cp_async_wait<0>();
     __syncthreads();
     for (int s = threadIdx.x; s < cnt; s += blockDim.x) {
       const int pos = p0 + s;
@@ -1972,9 +1973,11 @@ grad_kernel(GradArgs a, int conj_a) {
       if (DIM == 3) l2 = weights_rt_d<W>(a.s.u[2][pos], g, w2, d2) - o[2];
       float gr[3] = {0.f, 0.f, 0.f}, gi[3] = {0.f, 0.f, 0.f};
       if (DIM == 2) {
+#pragma unroll (W > 0 ? W : 1)
         for (int t0 = 0; t0 < w; ++t0) {
           const float2* row = tile + (l0 + t0) * g.pd[1] + l1;
           float sr = 0.f, si = 0.f, dr = 0.f, di = 0.f;
+#pragma unroll (W > 0 ? W : 1)
           for (int t1 = 0; t1 < w; ++t1) {
             float2 v = row[t1];
             sr = fmaf(w1[t1], v.x, sr);
@@ -1988,10 +1991,13 @@ grad_kernel(GradArgs a, int conj_a) {
           gi[1] = fmaf(w0[t0], di, gi[1]);
         }
       } else {
+#pragma unroll (W > 0 ? W : 1)
         for (int t0 = 0; t0 < w; ++t0) {
+#pragma unroll (W > 0 ? W : 1)
           for (int t1 = 0; t1 < w; ++t1) {
             const float2* row = tile + ((l0 + t0) * g.pd[1] + (l1 + t1)) * g.pd[2] + l2;
             float sr = 0.f, si = 0.f, dr = 0.f, di = 0.f;
+#pragma unroll (W > 0 ? W : 1)
             for (int t2 = 0; t2 < w; ++t2) {
               float2 v = row[t2];
               sr = fmaf(w2[t2], v.x, sr);
@@ -2030,7 +2036,8 @@ GBN_UNROLL
 // cotangents are summed per lane over all transforms and the lanes reduced once.
 // Bound by L1 and issue like interp_wc; against the tile kernel, which evaluates
 // the weights again for every transform and waits at its tile barriers: 131 072
-// samples, 8 transforms 166 -> 56 us.
+// samples, 8 transforms 166 -> 56 us.  Few transforms of many samples stay with the
+// tiles (dispatch_grad).
 // ---------------------------------------------------------------------------
 template <int W>
 __global__ void __launch_bounds__(GBN_THREADS, 4)
@@ -2176,7 +2183,8 @@ cudaError_t launch_grad_t(const GradArgs& a, int conj_a, cudaStream_t st) {
   auto k = grad_kernel<DIM, W>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  k<<<a.s.nsub, GBN_THREADS, smem, st>>>(a, conj_a);
+  // a thread a sample: subproblems of up to 128 leave half of 256 idle
+  k<<<a.s.nsub, a.s.maxsub <= 128 ? 128 : GBN_THREADS, smem, st>>>(a, conj_a);
   return cudaGetLastError();
 }
 
@@ -2319,12 +2327,30 @@ cudaError_t launch_grad_wc2d(const GradArgs& a, cudaStream_t st) {
 template <int DIM>
 cudaError_t dispatch_grad(const GradArgs& a, cudaStream_t st) {
   if constexpr (DIM == 2) {
-    if (a.g.w == 7) return launch_grad_wc2d<7>(a, st);
-    if (a.g.w == 6) return launch_grad_wc2d<6>(a, st);
-    if (a.g.w == 5) return launch_grad_wc2d<5>(a, st);
-    if (a.g.w == 4) return launch_grad_wc2d<4>(a, st);
+    // Straight from the grid, or from tiles, which read each cell once but evaluate the
+    // weights again for every transform: one, two or up to four transforms of enough
+    // samples, dense enough to share cells.  w = 7, us, grid / tiles: 128^2 images, 32 768
+    // radial samples, one transform 14 / 10, 1 M 234 / 57, two 251 / 142, four 291 / 262;
+    // 131 072, two 38 / 26, four 43 / 43; 1000^2, 131 072 uniform ones, one 39 / 39, two
+    // 45 / 144.
+    const int64_t M = a.s.M, G = a.g.G;
+    const bool tiles = a.ntr == 1   ? M >= 32768 && 16 * M >= G
+                       : a.ntr == 2 ? M >= 65536 && 3 * M >= G
+                                    : a.ntr <= 4 && M >= 524288 && 2 * M >= G;
+    if (!tiles) {
+      if (a.g.w == 7) return launch_grad_wc2d<7>(a, st);
+      if (a.g.w == 6) return launch_grad_wc2d<6>(a, st);
+      if (a.g.w == 5) return launch_grad_wc2d<5>(a, st);
+      if (a.g.w == 4) return launch_grad_wc2d<4>(a, st);
+    }
   }
-  // 3D and other widths: runtime-width tiles
+  // unrolled tiles: 3D, 8 transforms, 1 M samples on 256^3 cells 10.6 ms with the
+  // runtime-width kernel (16-entry arrays in local memory), 3.7 for w = 7; other widths
+  // take that one
+  if (a.g.w == 7) return launch_grad_t<DIM, 7>(a, a.conj_a, st);
+  if (a.g.w == 6) return launch_grad_t<DIM, 6>(a, a.conj_a, st);
+  if (a.g.w == 5) return launch_grad_t<DIM, 5>(a, a.conj_a, st);
+  if (a.g.w == 4) return launch_grad_t<DIM, 4>(a, a.conj_a, st);
   return launch_grad_t<DIM, 0>(a, a.conj_a, st);
 }
 
