@@ -2266,8 +2266,13 @@ cudaError_t dispatch_interp(const InterpArgs& a, cudaStream_t st) {
   // GBN_INTERP=tile forces tiles
   if (a.g.w == 7 && (a.g.method_interp == 4 || (DIM == 2 && a.g.method_interp == 0)))
     return launch_interp_wc_t<DIM>(a, st);
-  if constexpr (DIM == 2) {  // the widths of eps 1e-3 .. 1e-5
-    if (a.g.method_interp == 0) {
+  if constexpr (DIM == 2) {
+    // The widths of eps 1e-3 .. 1e-5; one transform of very many samples from tiles.  us,
+    // gather / tiles: w = 6 131 072 samples on 256^2 cells 21 / 25, 524 288 66 / 61, 2 M on
+    // 512^2 246 / 209; w = 5 262 144 on 128^2 32 / 33, 1 M 110 / 103; w = 4 524 288 52 / 53,
+    // 2 M 190 / 183.
+    const bool dense = a.ntr == 1 && a.s.M >= 2 * a.g.G && a.s.M >= (int64_t)1 << (24 - a.g.w);
+    if (a.g.method_interp == 0 && !dense) {
       if (a.g.w == 6) return launch_interp_wc_t<2, 6>(a, st);
       if (a.g.w == 5) return launch_interp_wc_t<2, 5>(a, st);
       if (a.g.w == 4) return launch_interp_wc_t<2, 4>(a, st);

@@ -50,3 +50,18 @@ def test_trajectory_gradient_from_tiles(gpu_pkg, eps, C, M):
         xn[:C], dn[:C] = x, dy
         out.append(op.plan.grad_traj_op(xn, None, dn, torch.empty(M, 2, device="cuda"), 1, n, 1.0).cpu())
     assert rel_l2(out[0], out[1]) < 2e-5
+
+
+@pytest.mark.parametrize("eps,M", [(1e-3, (1 << 20) - 1), (1e-3, 1 << 20), (1e-4, (1 << 19) - 1), (1e-4, 1 << 19),
+                                   (1e-5, (1 << 18) - 1), (1e-5, 1 << 18)])
+def test_one_transform_of_many_samples(gpu_pkg, monkeypatch, eps, M):
+    rng = np.random.default_rng(M)
+    shape = (50, 63)
+    k = rng.uniform(-0.5, 0.5, (M, 2)).astype(np.float32)
+    x = (rng.standard_normal((1, 1, *shape)) + 1j * rng.standard_normal((1, 1, *shape))).astype(np.complex64)
+    out = []
+    for interp in ("auto", "gm"):
+        monkeypatch.setenv("GBN_INTERP", interp)
+        op = gpu_pkg.MRIGB300(k, shape, squeeze_dims=False, eps=eps)
+        out.append(np.asarray(op.op(x)))
+    assert rel_l2(out[0], out[1]) < BOUND
