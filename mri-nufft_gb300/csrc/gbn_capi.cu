@@ -865,7 +865,7 @@ int gbn_plan_create(int dim, const int64_t* n_modes, double upsampfac, double ep
         int bs = dim == 2 ? binsz2[d] : binsz3[d];
         if (bs > nf) bs = (int)nf;
         g.bs[d] = bs;
-        g.nkey[d] = (int)nf + g.koff - w / 2;
+        g.nkey[d] = (int)nf;
         g.nb[d] = (g.nkey[d] + bs - 1) / bs;
         g.pd[d] = d == 2 ? (bs + w) & ~1 : bs + w - 1;  // 3D tile rows: even (pairs of cells)
         g.uscale[d] = (float)((double)nf / (2.0 * M_PI));

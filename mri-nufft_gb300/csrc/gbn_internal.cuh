@@ -29,7 +29,7 @@ struct Geom {
   int nb[3];     // number of bins per axis
   int pd[3];     // padded tile extent per axis: bs + w - 1, even along z (unused axes: 1)
   int nkey[3];   // sort keys per axis: a sample's key is its first footprint cell + koff
-  int koff;      // floor(w / 2) rounded up to even, so that even-sized bins start on even cells
+  int koff;      // floor(w / 2) rounded up to even: even-sized bins start on even cells
   int w;         // kernel width in cells
   float beta;    // ES shape parameter
   float halfw;   // w / 2
@@ -145,12 +145,13 @@ __device__ __forceinline__ float fold_coord(float k, float uscale, int nf) {
 }
 
 // Sort key of a folded coordinate, the first footprint cell + koff in
-// [0, nkey).  Samples whose footprint starts at nf - floor(w / 2) or later
-// move one period down (u in [-1, 0), an exact subtraction), so that every
-// footprint starts in [-floor(w / 2), nf - floor(w / 2)).
+// [0, nf).  Samples whose footprint starts at nf - koff or later move one
+// period down (u in [-2, 0), an exact subtraction; grids of one cell may take
+// two), so that every footprint starts in [-koff, nf - koff): as many keys as
+// cells, and bins of 8 divide axes that 8 divides.
 __device__ __forceinline__ int key_of(float& u, int nf, const Geom& g, int d) {
   int o = (int)ceilf(u - g.halfw);
-  if (o + (g.w >> 1) >= nf) {
+  for (int i = 0; i < 2 && o + g.koff >= nf; ++i) {
     u -= (float)nf;
     o = (int)ceilf(u - g.halfw);
   }
