@@ -189,7 +189,9 @@ int gbn_grad_traj_adj(gbn_plan plan, const void* dx, const void* smaps, const vo
  * (base.py:904-914, cufinufft.py:259-269).  Each stage of a batched op / adj
  * is ONE persistent launch of this library over a work table covering every
  * instance (pad, interp; zero, spread, crop), plus one cuFFT call per
- * instance.  Every plan needs gbn_setpts and ntrans >= its coil count.
+ * instance.  Every plan needs gbn_setpts and ntrans >= its coil count.  3D plans of
+ * several transforms should have bins of 8 cells (gbn_plan_tune): the bins they
+ * choose for their own kernels leave these ones without the row spreader.
  * gbn_batch_bind fixes the device buffers of every instance (image, coil maps
  * or NULL, k-space, density or NULL, scale, coil count) so that
  * gbn_batch_op / gbn_batch_adj take only a stream and can be captured in a

@@ -3,7 +3,8 @@
 For a problem class — (dim, image size, sampling density, coil count) — it
 times the candidate configurations on the instance's own trajectory (one
 forward + one adjoint of random data per candidate, CUDA events, best of a
-few repetitions) and keeps the fastest.  Results are cached in a JSON file
+few repetitions) and keeps the fastest; the plan's own choice comes first, so that tuning
+returns nothing slower.  Results are cached in a JSON file
 (``GBN_TUNE_CACHE`` or ``~/.cache/mrinufft_gb300/tune.json``) so a class is
 timed once per machine.  Sampling density is bucketed by powers of two of
 samples per fine-grid cell.
@@ -22,9 +23,9 @@ from .params import fine_shape
 from .plan import NufftPlan
 
 CANDIDATES = {
-    # "auto" is the dimension's default kernel (2D: warp-cooperative direct
-    # interpolation; 3D: shared-memory tiles); in 2D the bins set the sort
-    # order (locality) of the direct kernels
+    # "auto" is the plan's own choice of interpolation; in 2D the bins set the sort
+    # order (locality) of the direct kernels.  Bins other than the plan's own (OWN)
+    # leave the tensor-core kernels and the 2D tiles of several transforms.
     2: [
         {"bins": (32, 32), "interp": "auto", "maxsub": 512},
         {"bins": (16, 16), "interp": "auto", "maxsub": 512},
@@ -40,6 +41,10 @@ CANDIDATES = {
 }
 
 
+# the bins the plan chooses itself
+OWN = {"bins": None, "interp": "auto", "maxsub": 512}
+
+
 def default_cache_path() -> Path:
     env = os.environ.get("GBN_TUNE_CACHE")
     if env:
@@ -48,7 +53,11 @@ def default_cache_path() -> Path:
 
 
 class Autotuner:
-    def __init__(self, cache_path=None, reps=3, eps=1e-6, persist=True, interp_methods=None):
+    """``own``: the plan's own bins are a candidate (not for kernels that read the bins
+    another way, as those of persistent batches do)."""
+
+    def __init__(self, cache_path=None, reps=3, eps=1e-6, persist=True, interp_methods=None, own=True):
+        self.own = bool(own)
         self.path = Path(cache_path) if cache_path else default_cache_path()
         self.interp_methods = None if interp_methods is None else tuple(interp_methods)
         self.reps = reps
@@ -67,6 +76,8 @@ class Autotuner:
             G *= n
         bucket = int(round(math.log2(max(M, 1) / G))) if M > 0 else -99
         meth = "all" if self.interp_methods is None else "+".join(self.interp_methods)
+        if self.own:
+            meth += "+own"  # choices made before there was this candidate are not taken
         return (f"{len(shape)}d:{'x'.join(map(str, shape))}:dens2^{bucket}:c{C}:eps{self.eps:g}"
                 f":{meth}")
 
@@ -99,9 +110,10 @@ class Autotuner:
         key = self.key(shape, k.shape[0], C)
         if key in self.cache:
             c = self.cache[key]
-            return {"bins": tuple(c["bins"]), "interp": c["interp"], "maxsub": c["maxsub"]}
+            bins = None if c["bins"] is None else tuple(c["bins"])
+            return {"bins": bins, "interp": c["interp"], "maxsub": c["maxsub"]}
         timings = []
-        for cfg in CANDIDATES[len(shape)]:
+        for cfg in ([OWN] if self.own else []) + CANDIDATES[len(shape)]:
             if self.interp_methods is not None and cfg["interp"] not in self.interp_methods:
                 continue
             try:
@@ -110,7 +122,8 @@ class Autotuner:
                 continue
             timings.append((t, cfg))
         t, cfg = min(timings, key=lambda x: x[0])
-        self.cache[key] = {"bins": list(cfg["bins"]), "interp": cfg["interp"],
+        bins = None if cfg["bins"] is None else list(cfg["bins"])
+        self.cache[key] = {"bins": bins, "interp": cfg["interp"],
                            "maxsub": cfg["maxsub"], "ms": t,
                            "timings": {f"{c['bins']}/{c['interp']}": tt for tt, c in timings}}
         if self.persist:
