@@ -30,10 +30,6 @@ namespace {
 using namespace tc;
 
 constexpr int kThreads = 256;
-// mean number of truncated steps, weighted by how much of the sum they see: half
-// of the w x rows of a footprint
-constexpr float kSteps2 = 3.5f;
-
 // the epilogue of one value: scale, residual against the data, density
 __device__ __forceinline__ void store_value(const InterpArgs& a, int64_t oi, float dj, float2 r) {
   if (a.mode == INTERP_RESID) {
@@ -201,7 +197,10 @@ __global__ void __launch_bounds__(kThreads, 2) interp_tc2d_kernel(InterpArgs a, 
     const int j = on ? a.s.perm[p0 + m] : 0;
     const float dj = on && a.density ? a.density[j] : 1.f;
     const uint32_t tl = tm + ((uint32_t)(32 * (warp & 3)) << 16);
-    const float2 tr = make_float2(kSteps2 * kTrunc, kSteps2 * kTrunc);
+    // mean number of truncated steps, weighted by how much of the sum they see: half of
+    // the w x rows of a footprint
+    const float lost = 0.5f * (float)g.w * kTrunc;
+    const float2 tr = make_float2(lost, lost);
     for (int t0 = (warp >> 2) * (TG / 2); t0 < ((warp >> 2) + 1) * (TG / 2); t0 += 4) {
       if (c0 + t0 >= a.ntr) break;
       float d[2][4], e[2][4];
