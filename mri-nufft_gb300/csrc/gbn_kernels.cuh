@@ -2251,7 +2251,7 @@ cudaError_t dispatch_interp(const InterpArgs& a, cudaStream_t st) {
     // warp-cooperative kernel where the subproblems are full enough and enough to fill
     // the GPU (each CTA takes the transforms in turn).  us, tiles / gather: radial, 512^2
     // cells, 52 samples a subproblem, 2535 of them, 2 / 8 / 16 transforms 21 / 37 / 58 and
-    // 25 / 43 / 72; spiral, 768^2, 45, 2939 of them, 16 64 / 71; uniform samples, 512^2, 42,
+    // 25 / 43 / 72; spiral, 768^2, 42.7, 3060 of them, 16 63 / 71; uniform samples, 512^2, 41.8,
     // 4 / 16 27 / 65 and 24 / 60; 256^2, 53, 622 of them, 4 / 8 / 16 15 / 21 / 30 and
     // 14 / 19 / 31; 128^2, 56, 291 of them, 4 / 64 12 / 62 and 10 / 49.  1490 subproblems
     // (400^2, 54), a second round of CTAs that is mostly empty: 2 / 4 / 8 15 / 25 / 36 and
@@ -2259,7 +2259,7 @@ cudaError_t dispatch_interp(const InterpArgs& a, cudaStream_t st) {
     const int64_t ns = a.s.nsub;
     const bool few = a.s.M >= 50 * ns && ns >= 760 && (a.ntr == 2 || ns <= 1216 || ns >= 2128);
     if (a.g.tile2 && a.g.method_interp == 0 && a.ntr > 1 &&
-        (a.ntr > 8 ? a.s.M >= 44 * ns && ns >= 456 : few))
+        (a.ntr > 8 ? 2 * a.s.M >= 85 * ns && ns >= 456 : few))
       return a.ntr > 2 ? dispatch_interp_w<2, 4>(a, st) : dispatch_interp_w<2, 2>(a, st);
   }
   // the rest of 2D at w = 7 takes the warp-cooperative direct kernel, 3D tiles;
