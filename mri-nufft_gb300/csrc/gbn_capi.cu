@@ -632,7 +632,7 @@ void run_fft_crop(gbn_plan p, const CropArgs& a, int isign, cudaStream_t st) {
     Span span(p, GBN_STAGE_FFT, st);
     ck(launch_fft2d_adj(a, const_cast<float2*>(a.fine), p->twiddles(), isign, st),
        "fused transform + crop");
-    p->launches += a.smaps && a.ntr > 1 ? 3 : 2;
+    p->launches += a.ordered && a.smaps && a.ntr > 1 ? 3 : 2;
     return;
   }
   if (p->fft3d) {
@@ -1511,6 +1511,7 @@ void toep_apply(gbn_toep t, const void* img, const void* smaps, void* out, int B
                                 accumulate || c0 > 0, sc)
                     : crop_args(p, nullptr, o + (int64_t)c0 * g.Nimg, T, accumulate, sc);
     ca.dec[0] = ca.dec[1] = ca.dec[2] = nullptr;
+    ca.ordered = 1;
     if (p->fft3d && g.nf[0] == 256) {  // the x transforms and the multiply in one pass over the lines
       Span span(p, GBN_STAGE_FFT, st);
       ck(launch_fft3d_gram(pa, ca, t->K, p->twiddles(), st), "fused Toeplitz Gram");

@@ -10,9 +10,11 @@
 //           written; x lines of every y (mode entries in, all out).
 //   adjoint x lines of every y (all in, mode entries out); y lines of the
 //           x-mode rows (all in), crop fused into the stores: divide by
-//           phihat, scale, and for coil maps conj(s_c) v_c, left in the rows of
-//           the transform's own grid and summed over the coils in order by a
-//           pass of its own (one coil goes straight to the image).
+//           phihat, scale, and for coil maps conj(s_c) v_c: one coil straight
+//           to the image, several added to it with float2 atomics (the image
+//           is cleared first unless the call accumulates) or, where the call
+//           wants the same bits every time (ordered), left in the rows of the
+//           transform's own grid and summed in order by a pass of its own.
 //   Toeplitz Gram (512-point x axis): the op's y pass, one pass over the x lines
 //           doing the forward transform, the multiply by the real spectrum and
 //           the inverse transform, then the adjoint's y pass with the crop.
@@ -302,9 +304,9 @@ __global__ void __launch_bounds__(kT, kCtas<A>) f2_x_kernel(Lines2 a) {
 
 // ---------------------------------------------------------------- y lines, crop fused
 // blockIdx.x: 16 consecutive x image rows; blockIdx.y: transform.  SET: the y modes.
-// With coil maps and several transforms conj(s_c) v_c takes the place of the row's
-// first n1 cells, which this CTA alone reads, before its first store.
-template <int A, int SET>
+// ORDERED, conj(s_c) v_c takes the place of the row's first n1 cells, which this CTA
+// alone reads, before its first store (one coil: the image).
+template <int A, int SET, bool ORDERED>
 __global__ void __launch_bounds__(kT, kCtas<A>)
 f2_crop_y_kernel(CropArgs a, float2* fine, const float2* __restrict__ tw, int conj) {
   extern __shared__ float2 s_dyn[];
@@ -317,7 +319,8 @@ f2_crop_y_kernel(CropArgs a, float2* fine, const float2* __restrict__ tw, int co
   const int ix = blockIdx.x * kL + l;
   const bool valid = ix < n0;
   const int c = blockIdx.y;
-  float2* const in = fine + (int64_t)c * g.G + (int64_t)img_to_fine(valid ? ix : 0, n0, g.nf[0]) * (16 * A);
+  const int64_t frow = (int64_t)c * g.G + (int64_t)img_to_fine(valid ? ix : 0, n0, g.nf[0]) * (16 * A);
+  const float2* in = a.fine + frow;
   float2 x[A];
 #pragma unroll
   for (int q = 0; q < A; ++q) {
@@ -352,10 +355,15 @@ f2_crop_y_kernel(CropArgs a, float2* fine, const float2* __restrict__ tw, int co
       v = f2scale(v, a.dec[1] ? f0 * a.dec[1][i1] : f0);
       if (a.smaps) {
         const float2 s = a.smaps[(int64_t)c * g.Nimg + irow + i1];
-        v = make_float2(s.x * v.x + s.y * v.y, s.x * v.y - s.y * v.x);
-      }
-      if (a.smaps && a.ntr > 1) {
-        in[i1] = v;
+        const float2 p = make_float2(s.x * v.x + s.y * v.y, s.x * v.y - s.y * v.x);
+        if constexpr (!ORDERED) {
+          atomicAdd(a.out + irow + i1, p);
+        } else if (a.ntr > 1) {
+          fine[frow + i1] = p;
+        } else {
+          float2* dst = a.out + irow + i1;
+          *dst = a.accumulate ? f2add(p, *dst) : p;
+        }
       } else {
         float2* dst = a.out + (int64_t)c * g.Nimg + irow + i1;
         if (a.accumulate) v = f2add(v, *dst);
@@ -365,11 +373,12 @@ f2_crop_y_kernel(CropArgs a, float2* fine, const float2* __restrict__ tw, int co
   }
 }
 
-// The coils' products of a pass (see above), summed in order: the same bits in every
-// run, as the crop pass of the other grids gives them.  blockIdx.x: 256 pixels of the
-// image row blockIdx.y.  Bound by the read of what the crop has just left in L2.
-// Against atomics of the crop into a cleared image, Gram of 384^2 images (768^2 cells):
-// 16 coils 155 -> 157 us, 40 coils 415 -> 428, one coil 47 -> 44.
+// The coils' products of an ordered pass, summed as the crop pass of the other grids
+// does.  blockIdx.x: 256 pixels of the image row blockIdx.y.  Bound by the read of what
+// the crop has just left in L2.  The Toeplitz Gram, which has no other atomics, takes
+// it: 384^2 images (768^2 cells), 16 coils 155 -> 157 us, 40 415 -> 428 against atomics.
+// The adjoint's spreading adds with atomics anyway; 480 effective coils of 256^2 images
+// in passes of 64 4.65 against 4.73 ms for op + adj.
 __global__ void __launch_bounds__(kT) f2_coil_sum_kernel(CropArgs a, const float2* __restrict__ fine) {
   const Geom& g = a.g;
   const int i1 = blockIdx.x * kT + threadIdx.x, ix = blockIdx.y;
@@ -452,8 +461,10 @@ cudaError_t prepare_a() {
   };
   chk(set_smem(f2_pad_y_kernel<A, kHalf>, y_smem<A>()));
   chk(set_smem(f2_pad_y_kernel<A, kModes>, y_smem<A>()));
-  chk(set_smem(f2_crop_y_kernel<A, kHalf>, y_smem<A>()));
-  chk(set_smem(f2_crop_y_kernel<A, kModes>, y_smem<A>()));
+  chk(set_smem(f2_crop_y_kernel<A, kHalf, false>, y_smem<A>()));
+  chk(set_smem(f2_crop_y_kernel<A, kHalf, true>, y_smem<A>()));
+  chk(set_smem(f2_crop_y_kernel<A, kModes, false>, y_smem<A>()));
+  chk(set_smem(f2_crop_y_kernel<A, kModes, true>, y_smem<A>()));
   chk(set_smem(f2_x_kernel<A, kHalf, kAll, true>, x_smem<A>()));
   chk(set_smem(f2_x_kernel<A, kModes, kAll, true>, x_smem<A>()));
   chk(set_smem(f2_x_kernel<A, kAll, kHalf, true>, x_smem<A>()));
@@ -472,8 +483,10 @@ void pad_y_a(const PadArgs& pa, const float2* tw, int conj, cudaStream_t st) {
 template <int A>
 void crop_y_a(const CropArgs& ca, float2* fine, const float2* tw, int conj, cudaStream_t st) {
   const dim3 gy((ca.g.n[0] + kL - 1) / kL, ca.ntr);
-  if (ca.g.n[1] == 8 * A) f2_crop_y_kernel<A, kHalf><<<gy, kT, y_smem<A>(), st>>>(ca, fine, tw, conj);
-  else f2_crop_y_kernel<A, kModes><<<gy, kT, y_smem<A>(), st>>>(ca, fine, tw, conj);
+  const bool half = ca.g.n[1] == 8 * A, ordered = ca.smaps && (ca.ordered || ca.ntr == 1);
+  auto k = half ? (ordered ? f2_crop_y_kernel<A, kHalf, true> : f2_crop_y_kernel<A, kHalf, false>)
+                : (ordered ? f2_crop_y_kernel<A, kModes, true> : f2_crop_y_kernel<A, kModes, false>);
+  k<<<gy, kT, y_smem<A>(), st>>>(ca, fine, tw, conj);
 }
 template <int A>
 void x_lines_a(const Lines2& x, int ntr, bool in_prune, cudaStream_t st) {
@@ -505,8 +518,13 @@ void pad_y(const PadArgs& pa, const Twiddles& tw, int conj, cudaStream_t st) {
   with_axis(pa.g.nf[1], [&](auto A) { pad_y_a<decltype(A)::value>(pa, tw.t[1], conj, st); });
 }
 cudaError_t crop_y(const CropArgs& ca, float2* fine, const Twiddles& tw, int conj, cudaStream_t st) {
+  const bool sum = ca.smaps && ca.ntr > 1;
+  if (sum && !ca.ordered && !ca.accumulate) {
+    cudaError_t e = cudaMemsetAsync(ca.out, 0, sizeof(float2) * (size_t)ca.g.Nimg, st);
+    if (e != cudaSuccess) return e;
+  }
   with_axis(ca.g.nf[1], [&](auto A) { crop_y_a<decltype(A)::value>(ca, fine, tw.t[1], conj, st); });
-  if (ca.smaps && ca.ntr > 1)
+  if (sum && ca.ordered)
     f2_coil_sum_kernel<<<dim3((ca.g.n[1] + kT - 1) / kT, ca.g.n[0]), kT, 0, st>>>(ca, fine);
   return cudaGetLastError();
 }

@@ -25,6 +25,7 @@ struct CropArgs {
   float2* out;          // SENSE: one image; calibrationless: ntr images
   int ntr;
   int accumulate;       // out += result
+  int ordered;          // coils are summed in order (fused 2D transforms; the other crops always do)
   float scale;
 };
 
