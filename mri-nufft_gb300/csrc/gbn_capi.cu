@@ -569,13 +569,13 @@ bool tc_spread_pays(gbn_plan p, int ntr) {
   }
   if (ntr < 2) return false;
   // tiles take 12 ns each, 24 in groups of 32 transforms; a sample and transform 0.1 ns
-  // (w = 7, warp-cooperative) or 0.15 for 25 cells, in a chain of 0.35 or 3.5 us a transform
+  // for 7 x 7 cells (warp-cooperative, w = 4 to 7; per-sample 0.15 for 5 x 5), in a chain
+  // of 0.35 us a transform (3.5)
   const double tile = ntr > 16 ? 0.0244 * ((ntr + 31) / 32) : 0.0122;
   const double tc = 5.0 + tile * p->nsub_s + 5e-5 * M;
+  if (g.w >= 4) return tc < 6.0 + 0.35 * ntr + 1e-4 * (g.w / 7.0) * M * ntr;
   const double cells = g.w * g.w / 25.0;
-  const double chain = g.w == 7 ? 6.0 + 0.35 * ntr : 8.0 + 3.5 * ntr * cells;
-  const double work = g.w == 7 ? 1e-4 * M * ntr : 1.5e-4 * cells * M * ntr;
-  return tc < (g.w == 7 ? chain + work : std::fmax(chain, 8.0 + work));
+  return tc < std::fmax(8.0 + 3.5 * ntr * cells, 8.0 + 1.5e-4 * cells * M * ntr);
 }
 
 void run_spread(gbn_plan p, const SpreadArgs& a, cudaStream_t st) {

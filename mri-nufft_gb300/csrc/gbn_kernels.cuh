@@ -1874,15 +1874,17 @@ spread_gm_kernel(SpreadArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// Warp-cooperative spreading with global vector atomics (w = 7).  Eight lanes
+// Warp-cooperative spreading with global vector atomics (w <= 7).  Eight lanes
 // serve one sorted sample: lane l adds to the footprint cells at offset l of
 // the last axis, so each warp instruction issues the float2 reductions of
-// four samples onto 7 contiguous cells each (two 32-byte sectors per sample
-// instead of one sector per lane).
+// four samples onto W contiguous cells each (two 32-byte sectors per sample
+// instead of one sector per lane).  2D, w = 4 to 6, against per-sample atomics, whose
+// lanes meet on the same cells where the sort makes neighbours of samples with the same
+// first cell: 1 M samples on 256^2 cells, one transform, w = 5 243 -> 205 us, w = 6 348 ->
+// 266; 16 384 on 512^2, 12 -> 8, 14 -> 8.
 // ---------------------------------------------------------------------------
-template <int DIM>
+template <int DIM, int W = 7>
 __device__ __forceinline__ void spread_wc_body(const SpreadArgs& a, const int64_t warp_id) {
-  constexpr int W = 7;
   const Geom& g = a.g;
   const int lane = threadIdx.x & 31;
   const int q = lane >> 3, l = lane & 7;
@@ -1931,10 +1933,10 @@ __device__ __forceinline__ void spread_wc_body(const SpreadArgs& a, const int64_
   }
 }
 
-template <int DIM>
+template <int DIM, int W>
 __global__ void __launch_bounds__(GBN_THREADS, 4)
 spread_wc_kernel(SpreadArgs a) {
-  spread_wc_body<DIM>(a, ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  spread_wc_body<DIM, W>(a, ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
 }
 
 // ---------------------------------------------------------------------------
@@ -2297,21 +2299,32 @@ cudaError_t dispatch_interp(const InterpArgs& a, cudaStream_t st) {
 }
 
 
-template <int DIM>
+template <int DIM, int W = 7>
 cudaError_t launch_spread_wc_t(const SpreadArgs& a, cudaStream_t st) {
   if (a.s.M == 0) return cudaSuccess;
   const int64_t warps = (a.s.M + 3) / 4;
   const unsigned blocks = (unsigned)((warps * 32 + GBN_THREADS - 1) / GBN_THREADS);
-  spread_wc_kernel<DIM><<<blocks, GBN_THREADS, 0, st>>>(a);
+  spread_wc_kernel<DIM, W><<<blocks, GBN_THREADS, 0, st>>>(a);
   return cudaGetLastError();
 }
 
 template <int DIM>
 cudaError_t dispatch_spread(const SpreadArgs& a, cudaStream_t st) {
-  // 2D at w = 7 defaults to warp-cooperative atomics (2.5x the per-sample
-  // atomics); 3D to the row kernel
+  // 2D at w = 4 to 7 defaults to warp-cooperative atomics (w = 7: 2.5x the
+  // per-sample atomics); 3D to the row kernel
   if (a.g.w == 7 && (a.g.method_spread == 2 || (DIM == 2 && a.g.method_spread == 0)))
     return launch_spread_wc_t<DIM>(a, st);
+  if constexpr (DIM == 2) {
+    // One transform of half a million samples and more keeps the per-sample kernel where
+    // it is the faster one (1 M on 2000^2 cells, w = 4 100 us of 133, w = 5 140 of 146; on
+    // 512^2 113 of 122, 163 of 146; on 128^2 279 of 225).
+    const bool many = a.ntr == 1 && a.s.M >= (1 << 19);
+    if (a.g.method_spread == 0) {
+      if (a.g.w == 6) return launch_spread_wc_t<2, 6>(a, st);
+      if (a.g.w == 5 && !(many && a.s.M < a.g.G)) return launch_spread_wc_t<2, 5>(a, st);
+      if (a.g.w == 4 && !(many && a.s.M < 32 * a.g.G)) return launch_spread_wc_t<2, 4>(a, st);
+    }
+  }
   if (DIM == 3 && rows_fit(a.g) && a.g.method_spread != 1) {
     if (a.g.w == 7) return a.ntr > 1 ? launch_spread_rows_t<7, 2>(a, st) : launch_spread_rows_t<7, 1>(a, st);
     return a.ntr > 1 ? launch_spread_rows_t<0, 2>(a, st) : launch_spread_rows_t<0, 1>(a, st);

@@ -351,11 +351,10 @@ class MRIGB300(_Base):
     # = 268 MB).  op of a numpy image transforms the coils in groups and
     # copies each group's k-space into the page-locked result on a copy
     # stream while the GPU works on the next group (3D kooshball, 16 coils:
-    # 7.6 against 8.1 ms per call).  adj_op makes one call over all coils:
-    # its kernels need the k-space before they start, and group calls would
-    # cost more than the copy they hide (2.2 ms per 4-coil group against
-    # 2.0 ms per pass of one call, whose kernels stage each sample's geometry
-    # once for every coil).
+    # 5.6 against 6.1 ms per call).  adj_op makes one call over all coils: its
+    # kernels need the k-space before they start, and a group's coil sum would
+    # have to be added to the last one's image, which the library's adjoint does
+    # not do (four calls of 4 coils 5.11 ms, one of 16 4.89, the copy 1.27).
     HOST_OVERLAP_BYTES = 32 << 20
 
     def _host_groups(self):

@@ -82,8 +82,8 @@ class NufftPlan:
         return b.value
 
     # ---------------------------------------------------------------- tuning
-    # "auto": the default kernel of the dimension (2D: warp-cooperative direct,
-    # 3D: shared-memory tiles)
+    # "auto": what the plan chooses (2D: gather, tiles or tensor cores by samples and
+    # transforms, 3D: shared-memory tiles)
     METHODS = {"auto": 0, "direct": 1, "double_buffered": 3, "warp_direct": 4, "warp_tile": 5}
 
     def tune(self, bins=None, interp=None, maxsub_cap=0):
